@@ -498,12 +498,10 @@ def other_ops(device, peak, quick=False, shift=0):
         ms = _time_op(lambda: bulk_b200.stable_sort_by_key(k, v), prep=prep, reps=reps)
         ksz = k0.element_size()
         byts = 2 * n * (ksz + 4)
-        # LSD radix: one pass per key byte; a pass reads the keys (digit
-        # counts), then reads and writes keys and payloads (scatter), plus the
-        # digit counts (n / 4096 tiles x 256 u32) written, scanned and read
+        # LSD radix: the keys are read once for every pass's digit counts, then
+        # each pass (one per key byte) reads and writes keys and payloads
         passes = ksz
-        counts = (n + 4095) // 4096 * 256 * 4
-        moved = passes * (n * ksz + 2 * n * (ksz + 4) + 4 * counts)
+        moved = n * ksz + passes * 2 * n * (ksz + 4)
         res[f"sort_by_key_{tag}_u32_2^{26 - shift}"] = {
             "ms": ms, "GBps": byts / ms / 1e6, "frac_of_hbm": byts / ms / 1e6 / peak, "algorithmic_bytes": byts,
             "radix_passes": passes,

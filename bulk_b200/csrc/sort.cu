@@ -332,7 +332,7 @@ size_t merge_sort_ws_bytes_t(uint64_t n) {
 }
 
 // Which sort an array gets: one block-sort launch when it fits one block
-// tile (the radix sort's passes are 4 or 8 times three launches), the radix
+// tile (4 or 8 radix passes cost more than its merge rounds there), the radix
 // sort up to 2^30 elements, the merge sort above.
 template <typename K>
 bool use_radix(uint64_t n) {

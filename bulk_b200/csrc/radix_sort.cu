@@ -16,7 +16,8 @@
 // once: a tile is ranked by digit and staged in shared memory in digit order,
 // where its keys of a digit go follows from the counts and a look-back over
 // the groups of tiles before it, and each digit's run is written contiguously
-// to its position.
+// to its position.  Large arrays of 8-byte keys are sorted by their upper four
+// digits alone where those tell the keys apart well enough (RsPlanWs below).
 //
 // A single array of up to 131,072 keys is sorted instead by one launch of one
 // thread-block cluster whose CTAs exchange their digit counts through
@@ -407,42 +408,221 @@ __device__ __forceinline__ int rs_tile_count(const RsGroup<K, P> &g, uint64_t ba
   return base >= g.n ? 0 : (g.n - base) < (uint64_t)T ? (int)(g.n - base) : T;
 }
 
-// ---- digit counts of every pass in one read of the keys.
-// Counters are spread over COPIES columns by lane, so that no two lanes of a
-// warp (two, for 8-byte keys) ever meet in a bank, however the digits are
-// distributed; a CTA adds its sums to the array's counts when its run of
-// tiles leaves the array.  128 KB of counters, one CTA of 1024 threads an SM.
-// The kernel also clears the status rows that the first pass will publish in.
-constexpr int kRsHistThreads = 1024;
-template <typename K>
-constexpr int rs_hist_copies() {
-  return sizeof(K) == 4 ? 32 : 16;
-}
-template <typename K>
-constexpr size_t rs_hist_smem_bytes() {
-  return (size_t)rs_passes<K>() * kRsBins * rs_hist_copies<K>() * 4;
+// ---- 8-byte keys: the upper half of the digits first.
+//
+// A large array's 8-byte keys seldom agree in their upper 32 bits unless they
+// are drawn from few values.  Where they do not, four passes over the upper
+// digits leave only short runs of keys that agree there, in input order, and
+// one read of the keys finds and sorts those runs in place: half the passes.
+// A sample decides which of the two an array gets (rs_sample_kernel); every
+// kernel launched after it works the decision out (a kernel with nothing to
+// do leaves at once):
+//   full    the passes of digits 0-3 and 4-7
+//   upper   the passes of digits 4-7, then rs_fix_kernel
+//   rescue  rs_fix_kernel met a run longer than it sorts (the sample missed
+//           it): the passes of digits 0-3 and 4-7 follow.  The array then
+//           holds its keys in another order, but equal keys still in input
+//           order, so the result is the same.
+struct RsPlanWs {
+  unsigned int repeats;  // sampled keys whose upper half another one has
+  unsigned int zeros;    // sampled keys whose upper half is zero
+  unsigned int rescue;
+  unsigned int pad;
+};
+enum RsPlan { kPlanFull, kPlanUpper, kPlanRescue };
+
+constexpr int kRsSampleThreads = 512, kRsSampleCtas = 32, kRsSamples = kRsSampleThreads * kRsSampleCtas;
+constexpr int kRsSampleSlots = 65536;
+constexpr uint32_t kRsSampleWindow = 65536;   // keys a CTA samples from
+// From here on arrays are planned.  u64/u32 on a B200, planned / all eight
+// passes: random keys 2^20 128 / 128 us, 2^22 218 / 300, 2^25 1060 / 1801,
+// 2^26 2009 / 3500; keys of 1000 values (the plan is all passes, and the idle
+// launches are lost) 2^20 159 / 118, 2^22 292 / 250, 2^25 1576 / 1533.
+constexpr uint64_t kRsPlanMinN = 1ull << 22;
+
+// A key's run has on average 1 + n * sum(p^2) keys (p the shares of the upper
+// halves' values), of which the sample's repeats estimate 2 * repeats /
+// samples^2: the upper digits alone are sorted by up to an average of about 8.
+__device__ __forceinline__ RsPlan rs_plan(const RsPlanWs *plan, uint64_t n) {
+  if (plan == nullptr) return kPlanFull;
+  const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(plan));
+  if (w.z != 0u) return kPlanRescue;
+  return (uint64_t)w.x * n <= 4ull * kRsSamples * kRsSamples ? kPlanUpper : kPlanFull;
 }
 
-template <typename K, typename P, typename Src, int C>
-__global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid_constant__ Src src,
-                                                                    unsigned int groups, unsigned int *hist,
-                                                                    uint4 *status) {
-  constexpr int COPIES = rs_hist_copies<K>(), BINS = rs_passes<K>() * kRsBins, PASSES = rs_passes<K>();
+// The digit that launch `launch` of an array's passes (three blocks of four)
+// sorts by, -1 for none; without a plan launch i sorts by digit i.
+__device__ __forceinline__ int rs_launch_digit(int launch, const RsPlanWs *plan, uint64_t n) {
+  if (plan == nullptr) return launch;
+  const RsPlan p = rs_plan(plan, n);
+  const int block = launch >> 2, i = launch & 3;
+  if (p == kPlanFull) return block < 2 ? launch : -1;
+  if (p == kPlanUpper) return block == 0 ? 4 + i : -1;
+  return block == 1 ? i : 4 + i;
+}
+
+// Every CTA takes one key from each 128th of a random window of 65,536 keys
+// and enters its upper half in a table of values seen (zeroed before; a zero
+// half is counted apart).  Windows, because reading 16,384 keys all over 2^26
+// costs their address translation; 128 keys apart, so that a sorted array's
+// runs that are short enough to be sorted in place rarely count.
+template <typename K>
+__global__ void __launch_bounds__(kRsSampleThreads) rs_sample_kernel(const K *keys, uint32_t n, unsigned int *table,
+                                                                     RsPlanWs *plan) {
+  constexpr uint32_t STRIDE = kRsSampleWindow / kRsSampleThreads;
+  auto mixed = [](unsigned int x) {
+    unsigned int h = (x + 1u) * 0x9e3779b1u;
+    h = (h ^ (h >> 15)) * 0x85ebca6bu;
+    h = (h ^ (h >> 13)) * 0xc2b2ae35u;
+    return h ^ (h >> 16);
+  };
+  const unsigned int me = blockIdx.x * kRsSampleThreads + threadIdx.x;
+  const uint64_t window = (uint64_t)mixed(blockIdx.x) * (n - kRsSampleWindow) >> 32;
+  const uint32_t at_key = threadIdx.x * STRIDE + mixed(me + kRsSampleCtas) % STRIDE;
+  const unsigned int up = (unsigned int)(RadixKey<K>::to(keys[window + at_key]) >> 32);
+  bool repeat = false;
+  if (up == 0u) {
+    repeat = atomicAdd(&plan->zeros, 1u) != 0u;
+  } else {
+    unsigned int at = (up * 0x9e3779b1u) / (unsigned int)(0x100000000ull / kRsSampleSlots);
+    for (int probe = 0; probe < kRsSamples; ++probe) {  // ends before: a quarter of the slots are taken at most
+      const unsigned int was = atomicCAS(table + at, 0u, up);
+      repeat = was == up;
+      if (was == 0u || repeat) break;
+      at = (at + 1) & (kRsSampleSlots - 1);
+    }
+  }
+  const int repeats = __syncthreads_count(repeat);
+  if (threadIdx.x == 0 && repeats != 0) atomicAdd(&plan->repeats, (unsigned int)repeats);
+}
+
+// Sorts every run of keys with equal upper halves (all of them in input order
+// within a run) by the lower halves, in place.  A warp sorts the runs that
+// start in its chunk of keys, which may reach into the kRsFixHalo keys after
+// it; the warp there sees that its first keys belong to an earlier run (their
+// upper halves do not change) and leaves them alone.  A key's place in its
+// run is the number of keys before it with a lower half not above its own
+// plus the number after it with one below: runs are a few keys long, and a
+// key without equal neighbours costs two comparisons.  A run longer than
+// kRsFixHalo is left as it is, and unless it is in order already (one value
+// many times) the array is sent to the rescue passes.  One read of the keys,
+// bound by memory where runs are rare; warps work on their own, so that one
+// warp's loads run behind another's comparisons (a CTA-wide tile of 4096 keys
+// between barriers took 271 us for 2^26 random keys on a B200).
+constexpr int kRsFixThreads = 128, kRsFixPer = 8, kRsFixChunk = 32 * kRsFixPer, kRsFixHalo = 64;
+
+template <typename K, typename P>
+__global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *vals, uint32_t n, RsPlanWs *plan) {
+  constexpr int WARPS = kRsFixThreads / 32, LEN = kRsFixChunk + kRsFixHalo, PER = LEN / 32;
+  using V = typename std::conditional<has_payload<P>(), P, char>::type;
+  if (rs_plan(plan, n) == kPlanFull) return;
+  // the keys' halves (up[-1]: of the key before the chunk); later, in the same
+  // place, the keys that move, at their new places
+  __shared__ uint64_t s_halves[WARPS][LEN + 1];
+  __shared__ uint16_t s_to[WARPS][LEN];  // where a key that moves goes
+  __shared__ V s_val[WARPS][has_payload<P>() ? LEN : 1];  // the payloads of the keys that move
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned int *low = reinterpret_cast<unsigned int *>(s_halves[warp]), *up = low + LEN + 1;
+  K *moved = reinterpret_cast<K *>(s_halves[warp]);
+  const uint64_t step = (uint64_t)gridDim.x * WARPS * kRsFixChunk;
+  for (uint64_t base = ((uint64_t)blockIdx.x * WARPS + warp) * kRsFixChunk; base < n; base += step) {
+    const int len = (int)((n - base) < (uint64_t)LEN ? (n - base) : (uint64_t)LEN);
+    const bool open = base + (uint64_t)len < n;  // keys follow the halo
+    K *const kp = keys + base;
+    {
+      K k[PER];
+#pragma unroll
+      for (int j = 0; j < PER; ++j)
+        if (j * 32 + lane < len) k[j] = kp[j * 32 + lane];
+      if (lane == 0) {
+        const unsigned int u = (unsigned int)(RadixKey<K>::to(base > 0 ? kp[-1] : k[0]) >> 32);
+        up[-1] = base > 0 ? u : ~u;
+      }
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        if (j * 32 + lane < len) {
+          const uint64_t u = RadixKey<K>::to(k[j]);
+          low[j * 32 + lane] = (unsigned int)u;
+          up[j * 32 + lane] = (unsigned int)(u >> 32);
+        }
+      }
+    }
+    __syncwarp();
+    unsigned int todo = 0;  // bit j: key j * 32 + lane has an equal neighbour
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = j * 32 + lane;
+      if (i < len && (up[i - 1] == up[i] || (i + 1 < len && up[i + 1] == up[i]))) todo |= 1u << j;
+    }
+    unsigned int moves = 0;
+    while (todo != 0) {
+      const int j = __ffs(todo) - 1, i = j * 32 + lane;
+      todo &= todo - 1;
+      const unsigned int u = up[i], l = low[i];
+      int first = i, last = i, rank = 0;  // the run is [first, last]
+      while (first > 0 && last - first < kRsFixHalo && up[first - 1] == u) {
+        --first;
+        rank += low[first] <= l;
+      }
+      // another warp's: it begins before the chunk, or in the halo
+      if ((first == 0 && up[-1] == u) || first >= kRsFixChunk) continue;
+      while (last - first < kRsFixHalo && last + 1 < len && up[last + 1] == u) {
+        ++last;
+        rank += low[last] < l;
+      }
+      if (last - first >= kRsFixHalo || (open && last + 1 == len)) {
+        if (i > first && low[i - 1] > l) plan->rescue = 1u;
+      } else if (first + rank != i) {
+        s_to[warp][i] = (uint16_t)(first + rank);
+        moves |= 1u << j;
+      }
+    }
+    if (__any_sync(0xffffffffu, moves != 0)) {
+      // the places that keys leave are the places that keys take
+      __syncwarp();
+      for (unsigned int m = moves; m != 0; m &= m - 1) {
+        const int i = (__ffs(m) - 1) * 32 + lane, to = s_to[warp][i];
+        moved[to] = kp[i];
+        if constexpr (has_payload<P>()) s_val[warp][to] = vals[base + i];
+      }
+      __syncwarp();  // everything is read before anything is written
+      for (unsigned int m = moves; m != 0; m &= m - 1) {
+        const int i = (__ffs(m) - 1) * 32 + lane;
+        kp[i] = moved[i];
+        if constexpr (has_payload<P>()) vals[base + i] = s_val[warp][i];
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ---- digit counts of every pass in one read of the keys.
+// Counters are spread over columns by lane, so that no two lanes of a warp
+// (two, where eight digits are counted) ever meet in a bank, however the
+// digits are distributed; a CTA adds its sums to the array's counts when its
+// run of tiles leaves the array.  128 KB of counters, one CTA of 1024 threads
+// an SM.  With a plan the first launch counts the digits that the passes
+// after it need and a second one, for the rescue, the rest.  The first also
+// clears the status rows that the first pass will publish in.
+constexpr int kRsHistThreads = 1024;
+constexpr size_t kRsHistSmemBytes = 128 * 1024;
+
+// Counts digits [FIRST, FIRST + DIGITS).
+template <typename K, typename P, typename Src, int C, int FIRST, int DIGITS>
+__device__ __forceinline__ void rs_count_digits(const Src &src, unsigned int groups, unsigned int *hist) {
+  constexpr int BINS = DIGITS * kRsBins, COPIES = (int)(kRsHistSmemBytes / 4) / BINS;
   constexpr int TILE = RsCfg<K, P>::TILE;
   constexpr int VEC = 16 / (int)sizeof(K), UNROLL = 4;
   extern __shared__ __align__(16) unsigned int rs_hist_smem[];
   const int tid = threadIdx.x, lane = tid & 31;
   for (int i = tid; i < BINS * COPIES / 4; i += kRsHistThreads)
     reinterpret_cast<uint4 *>(rs_hist_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (uint64_t i = (uint64_t)blockIdx.x * kRsHistThreads + tid; i < (uint64_t)groups * (kRsBins / 4);
-       i += (uint64_t)gridDim.x * kRsHistThreads)
-    status[i] = make_uint4(0u, 0u, 0u, 0u);
   unsigned int *col = rs_hist_smem + (lane & (COPIES - 1));
   auto add = [&](K key) {
     const auto u = RadixKey<K>::to(key);
 #pragma unroll
-    for (int p = 0; p < PASSES; ++p)
-      atomicAdd(col + (p * kRsBins + (int)((u >> (8 * p)) & 0xffu)) * COPIES, 1u);
+    for (int p = 0; p < DIGITS; ++p)
+      atomicAdd(col + (p * kRsBins + (int)((u >> (8 * (FIRST + p))) & 0xffu)) * COPIES, 1u);
   };
   const uint64_t tiles = (uint64_t)groups * C;
   uint64_t t = tiles * blockIdx.x / gridDim.x;
@@ -482,7 +662,7 @@ __global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid
       for (uint64_t i = head + nv * VEC + tid; i < cnt; i += kRsHistThreads) add(p[i]);
     }
     __syncthreads();
-    unsigned int *out = hist + (uint64_t)gr.array * BINS;
+    unsigned int *out = hist + ((uint64_t)gr.array * rs_passes<K>() + FIRST) * kRsBins;
     for (int b = tid; b < BINS; b += kRsHistThreads) {
       unsigned int sum = 0;
 #pragma unroll 8
@@ -496,6 +676,24 @@ __global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid
     __syncthreads();
     t += take;
   }
+}
+
+template <typename K, typename P, typename Src, int C>
+__global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid_constant__ Src src,
+                                                                    unsigned int groups, unsigned int *hist,
+                                                                    uint4 *status, const RsPlanWs *plan,
+                                                                    bool rescue) {
+  const RsPlan p = rs_plan(plan, plan != nullptr ? src.group(0).n : 0);
+  if (rescue) {
+    if (p == kPlanRescue) rs_count_digits<K, P, Src, C, 0, 4>(src, groups, hist);
+    return;
+  }
+  for (uint64_t i = (uint64_t)blockIdx.x * kRsHistThreads + threadIdx.x; i < (uint64_t)groups * (kRsBins / 4);
+       i += (uint64_t)gridDim.x * kRsHistThreads)
+    status[i] = make_uint4(0u, 0u, 0u, 0u);
+  if constexpr (sizeof(K) == 4) rs_count_digits<K, P, Src, C, 0, 4>(src, groups, hist);
+  else if (p == kPlanFull) rs_count_digits<K, P, Src, C, 0, 8>(src, groups, hist);
+  else rs_count_digits<K, P, Src, C, 4, 4>(src, groups, hist);
 }
 
 // ---- one pass: stable scatter by digit (keys -> temporaries on even passes,
@@ -647,7 +845,7 @@ __device__ __forceinline__ void rs_scout(const Src &src, int pass, unsigned int 
 
 template <typename K, typename P, typename Src, int C>
 __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_BLOCKS)) rs_pass_kernel(
-    const __grid_constant__ Src src, int pass, unsigned int groups, const unsigned int *hist, unsigned int *tickets,
+    const __grid_constant__ Src src, int launch, const RsPlanWs *plan, unsigned int groups, const unsigned int *hist, unsigned int *tickets,
     unsigned int *status, unsigned int *status_next, WsHeader *hdr, unsigned int ahead, unsigned long long limit_ns) {
   using Cfg = RsCfg<K, P>;
   constexpr int ITEMS = Cfg::ITEMS, WARPS = Cfg::WARPS, THREADS = Cfg::THREADS, TILE = Cfg::TILE;
@@ -670,7 +868,9 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   __shared__ __align__(8) uint64_t s_group_bar;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned int me = rs_cluster_rank();
-  const bool odd = pass & 1;
+  const int pass = rs_launch_digit(launch, plan, plan != nullptr ? src.group(0).n : 0);  // the digit
+  if (pass < 0) return;
+  const bool odd = launch & 1;
   const RsRanker ranker(s_table[warp], s_bits[warp]);
 
   auto elem = [&](int j) { return warp * 32 * ITEMS + j * 32 + lane; };
@@ -678,7 +878,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   auto load_keys = [&](const RsGroup<K, P> &gr) {
     const uint64_t base = ((uint64_t)gr.local * C + me) * TILE;
     const int count = rs_tile_count(gr, base);
-    const K *in = (odd ? gr.tk : (pass == 0 ? gr.src_k : gr.keys)) + base + elem(0);
+    const K *in = (odd ? gr.tk : (launch == 0 ? gr.src_k : gr.keys)) + base + elem(0);
     if (count == TILE) {
 #pragma unroll
       for (int j = 0; j < ITEMS; ++j) k[j] = in[j * 32];
@@ -710,7 +910,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   rs_cluster_sync();  // every CTA of the cluster runs, its barriers ready, before anything is sent to it
   if (me == 0 && warp == 0) {
     unsigned int t = 0;
-    if (lane == 0) t = atomicAdd(&tickets[pass], 1u);
+    if (lane == 0) t = atomicAdd(&tickets[launch], 1u);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (lane < C) rs_push_u32(&s_group, t, &s_group_bar, (uint32_t)lane);
   }
@@ -745,16 +945,16 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
         mbar_arrive_expect_tx(&s_base_bar[par], BASE_TX);
       }
       unsigned int ticket = groups;
-      if (more && me == 0 && tid == 0) ticket = atomicAdd(&tickets[pass], 1u);
+      if (more && me == 0 && tid == 0) ticket = atomicAdd(&tickets[launch], 1u);
       if (tid == THREADS - 1 && ahead != 0 && g + ahead < groups) {
         // into L2: the tile of a group that a cluster will take about an iteration from now
         const RsGroup<K, P> f = src.group(g + ahead);
         const uint64_t base = ((uint64_t)f.local * C + me) * TILE;
         const uint64_t fc = (uint64_t)rs_tile_count(f, base);
         if (fc > 0) {
-          prefetch_l2_range((odd ? f.tk : (pass == 0 ? f.src_k : f.keys)) + base, fc * sizeof(K));
+          prefetch_l2_range((odd ? f.tk : (launch == 0 ? f.src_k : f.keys)) + base, fc * sizeof(K));
           if constexpr (has_payload<P>())
-            prefetch_l2_range((odd ? f.tv : (pass == 0 ? f.src_v : f.vals)) + base, fc * sizeof(P));
+            prefetch_l2_range((odd ? f.tv : (launch == 0 ? f.src_v : f.vals)) + base, fc * sizeof(P));
         }
       }
       // ---- digits and ranks.  Past the tile's end the digit is 255: those
@@ -797,7 +997,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
       }
       // payloads on their way
       if constexpr (has_payload<P>()) {
-        const P *in = (odd ? gr.tv : (pass == 0 ? gr.src_v : gr.vals)) + tbase + elem(0);
+        const P *in = (odd ? gr.tv : (launch == 0 ? gr.src_v : gr.vals)) + tbase + elem(0);
         if (count == TILE) {
 #pragma unroll
           for (int j = 0; j < ITEMS; ++j) v[j] = in[j * 32];
@@ -1074,11 +1274,11 @@ inline int rs_group_ctas(const uint64_t *sizes, uint32_t count) {
 
 // Workspace (after the 256-byte header): every array's key and payload
 // temporaries; zeroed before each sort: the arrays' digit counts and the
-// passes' tickets; two buffers of status rows (one word a digit and group),
+// passes' tickets and a planned sort's sample; two buffers of status rows (one word a digit and group),
 // of which each pass publishes in one and clears the other.
 template <typename K, typename P>
 struct RsLayout {
-  size_t tmp, hist, tickets, zero_bytes, status[2], total;
+  size_t tmp, hist, tickets, plan, samples, zero_bytes, status[2], total;
   uint64_t groups;
   int ctas;
   RsLayout(const uint64_t *sizes, uint32_t count) {
@@ -1094,7 +1294,10 @@ struct RsLayout {
     hist = o;
     o += (size_t)count * rs_passes<K>() * kRsBins * 4;
     tickets = o;
+    plan = o + 128;
     o += 256;
+    samples = o;
+    if (sizeof(K) == 8 && count == 1 && sizes[0] >= kRsPlanMinN) o += (size_t)kRsSampleSlots * 4;
     zero_bytes = o - hist;
     for (size_t &s : status) {
       s = o;
@@ -1140,13 +1343,15 @@ struct RsPassConfig {
 // The passes over `src` (one array or a batch).
 template <typename K, typename P, typename Src, int C>
 int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream_t stream) {
+  // one array of 8-byte keys: see RsPlanWs
+  constexpr bool kPlanned = sizeof(K) == 8 && std::is_same<Src, RsOne<K, P>>::value;
   int st;
   auto hist_kern = rs_hist_kernel<K, P, Src, C>;
   auto pass_kern = rs_pass_kernel<K, P, Src, C>;
   struct HistSite {};
   struct PassSite {};
   host::KernelSetup hs;
-  if ((st = host::kernel_setup<HistSite>(hist_kern, kRsHistThreads, rs_hist_smem_bytes<K>(), &hs)) != BK_OK) return st;
+  if ((st = host::kernel_setup<HistSite>(hist_kern, kRsHistThreads, kRsHistSmemBytes, &hs)) != BK_OK) return st;
   int clusters = 0;  // resident at once
   st = host::once_per_device<PassSite>(&clusters, [&](int *out) -> int {
     int e = host::set_smem_attrs(pass_kern, rs_smem_bytes<K, P>());
@@ -1163,21 +1368,46 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
   const host::DebugFault df = host::debug_fault();
   const unsigned long long limit = df.spin_limit_ns ? df.spin_limit_ns : host::kDefaultSpinLimitNs;
   if ((st = host::from_cuda(cudaMemsetAsync(hist, 0, L.zero_bytes, stream))) != BK_OK) return st;
+  RsPlanWs *plan = nullptr;
+  int fix_ctas = 0;
+  if constexpr (kPlanned) {
+    if (src.n >= kRsPlanMinN) {
+      plan = reinterpret_cast<RsPlanWs *>(ws + L.plan);
+      struct FixSite {};
+      host::KernelSetup fs;
+      if ((st = host::kernel_setup<FixSite>(rs_fix_kernel<K, P>, kRsFixThreads, 0, &fs)) != BK_OK) return st;
+      fix_ctas = (int)fs.resident_ctas;
+      rs_sample_kernel<K><<<kRsSampleCtas, kRsSampleThreads, 0, stream>>>(
+          src.keys, (uint32_t)src.n, reinterpret_cast<unsigned int *>(ws + L.samples), plan);
+      if ((st = host::launch_status()) != BK_OK) return st;
+    }
+  }
   const uint64_t tiles = L.groups * C;
   const unsigned hist_ctas = (unsigned)(tiles < hs.resident_ctas ? tiles : hs.resident_ctas);
-  hist_kern<<<hist_ctas, kRsHistThreads, rs_hist_smem_bytes<K>(), stream>>>(
-      src, groups, hist, reinterpret_cast<uint4 *>(ws + L.status[0]));
+  hist_kern<<<hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream>>>(
+      src, groups, hist, reinterpret_cast<uint4 *>(ws + L.status[0]), plan, false);
   if ((st = host::launch_status()) != BK_OK) return st;
   const unsigned used = groups < (unsigned)clusters ? groups : (unsigned)clusters;
   RsPassConfig<K, P, C> pc(used, stream);
   // L2 prefetch distance: the table's number of residencies ahead (0: none)
   const tune::Knobs kn = tune::knobs_for(tune::kSort, RsCfg<K, P>::BYTES, L.groups * C * RsCfg<K, P>::TILE);
   const unsigned ahead = used * (unsigned)kn.prefetch;
-  for (int p = 0; p < rs_passes<K>(); ++p) {
-    st = host::from_cuda(cudaLaunchKernelEx(&pc.cfg, pass_kern, src, p, groups, (const unsigned int *)hist, tickets,
+  const int launches = plan != nullptr ? 12 : rs_passes<K>();
+  for (int p = 0; p < launches; ++p) {
+    st = host::from_cuda(cudaLaunchKernelEx(&pc.cfg, pass_kern, src, p, (const RsPlanWs *)plan, groups,
+                                            (const unsigned int *)hist, tickets,
                                             reinterpret_cast<unsigned int *>(ws + L.status[p & 1]),
                                             reinterpret_cast<unsigned int *>(ws + L.status[(p & 1) ^ 1]), hdr, ahead, limit));
     if (st != BK_OK) return st;
+    if constexpr (kPlanned) {
+      if (plan != nullptr && p == 3) {
+        rs_fix_kernel<K, P><<<fix_ctas, kRsFixThreads, 0, stream>>>(src.keys, src.vals, (uint32_t)src.n, plan);
+        if ((st = host::launch_status()) != BK_OK) return st;
+        hist_kern<<<hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream>>>(
+            src, groups, hist, reinterpret_cast<uint4 *>(ws + L.status[0]), plan, true);
+        if ((st = host::launch_status()) != BK_OK) return st;
+      }
+    }
   }
   return BK_OK;
 }

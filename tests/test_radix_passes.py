@@ -67,3 +67,43 @@ def test_batches_with_full_and_ragged_groups(cuda, key, value, many):
         _check(k, v, gk, gv)
         assert np.array_equal(host(sk), k)
     assert bulk_b200.workspace_status() == 0
+
+
+# ---- 8-byte keys from 2^22 on: upper digits first, then the short runs that agree there
+PLAN_MIN = 1 << 22
+
+
+def _wide(tag, kind, n, rng):
+    full = rng.integers(0, 1 << 64, n, dtype=np.uint64)
+    if kind == "runs of a few":      # about eight keys an upper half
+        k = (rng.integers(0, n // 8, n, dtype=np.uint64) << np.uint64(32)) | (full & np.uint64(0xFF))
+    elif kind == "few upper halves":  # the sample sends it to all eight passes
+        k = (rng.integers(0, 1000, n, dtype=np.uint64) << np.uint64(40)) | (full & np.uint64(0xFFFFFF))
+    elif kind in ("long run", "longest run"):  # too long to sort in place, too rare for the sample
+        k = full.copy()
+        at = n // 3 + (np.arange(400) if kind == "long run" else np.arange(256))
+        k[at] = (np.uint64(77) << np.uint64(32)) | (full[at] & np.uint64(0xF))
+    else:
+        k = full
+    if tag == "f64":
+        k = k.copy()
+        k[(k >> np.uint64(52) & np.uint64(0x7FF)) == 0x7FF] = 0x3FF0000000000000  # no NaN
+        k[::1000] = 0x8000000000000000
+        k[1::1000] = 0  # the two zeros tie
+    return k.view(NP[tag])
+
+
+@pytest.mark.parametrize("kind", ["full", "runs of a few", "few upper halves", "long run", "longest run"])
+@pytest.mark.parametrize("key,value", [("u64", "u32"), ("i64", None), ("f64", "u64")])
+def test_wide_keys_by_upper_digits(cuda, key, value, kind):
+    rng = np.random.default_rng(7)
+    for n in (PLAN_MIN, PLAN_MIN + 4097):
+        keys = _wide(key, kind, n, rng)
+        if value is None:
+            _check(keys, None, bulk_b200.stable_sort_by_key(dev(keys)), None)
+        else:
+            vals = np.arange(n, dtype=NP[value])
+            gk, gv = bulk_b200.stable_sort_by_key(dev(keys), dev(vals))
+            _check(keys, vals, gk, gv)
+            assert np.array_equal(host(gk).view(np.uint64), keys[np.argsort(keys, kind="stable")].view(np.uint64))
+        assert bulk_b200.workspace_status() == 0

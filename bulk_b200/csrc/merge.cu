@@ -6,18 +6,19 @@
 // merge.cu:12-97), which is keys-only; the by-key form follows the bounded
 // group merge_by_key (bulk/algorithm/merge.hpp:507-607).
 //
-// Here: a partition kernel computes the A/B split at every tile boundary;
-// then persistent CTAs merge 4096-output tiles (2048 for 8-byte keys) in a
-// two-buffer pipeline.  A loader lane brings a tile's A and B key and
-// payload ranges into shared memory with untiled bulk (TMA) copies -- each
-// range widened to whole 16-byte chunks, the ragged ends by plain loads --
-// while the compute warps merge the previous tile: each thread finds its
-// diagonal with a merge-path search in shared memory, merges its outputs
-// serially (branch-free: keys plus the shared-memory index of each output's
-// source, which gathers the payload), and, once every thread has read its
-// inputs, writes them back in place in the 128-byte-swizzled layout; the
-// loader then stores the tile with tiled tensor copies, which undo the
-// swizzle.  No thread loads or stores a tile element itself on this path.
+// Here: persistent CTAs merge runs of 4096-output tiles (2048 for 8-byte keys)
+// in a two-buffer pipeline.  A tile's A/B split comes from a partition kernel
+// where a CTA has many tiles, and from the CTA's loader warp otherwise.  The
+// loader's first lane brings a tile's A and B key and payload ranges into
+// shared memory with untiled bulk (TMA) copies -- each range widened to whole
+// 16-byte chunks, the ragged ends by plain loads -- while the compute warps
+// merge the previous tile: each thread finds its diagonal with a merge-path
+// search in shared memory, merges its outputs serially (branch-free: keys plus
+// the shared-memory index of each output's source, which gathers the payload),
+// and, once every thread has read its inputs, writes them back in place in the
+// 128-byte-swizzled layout; the loader then stores the tile with tiled tensor
+// copies, which undo the swizzle.  No thread loads or stores a tile element
+// itself on this path.
 #include <algorithm>
 
 #include "bk_common.cuh"
@@ -68,6 +69,36 @@ __global__ void merge_partition_kernel(const K *a, uint64_t na, const K *b, uint
   parts[k] = merge_path<K, uint64_t>(a, na, b, nb, diag);
 }
 
+// The number of A elements among the first `diag` outputs, known to lie in
+// [lo, hi]: the first mid there with b[diag - 1 - mid] < a[mid] (ties go to A).
+// The whole warp searches: each round its lanes cut the range into 65 parts
+// with two probes each, so a tile's 4097 candidates take two rounds of loads
+// and 2^26 take five, where a one-thread binary search waits for 12 or 26 one
+// after another.
+template <typename K>
+__device__ __forceinline__ uint64_t merge_split_warp(const K *a, const K *b, uint64_t diag, uint64_t lo, uint64_t hi,
+                                                     int lane) {
+  while (lo < hi) {
+    const uint64_t step = (hi - lo + 64) / 65;
+    const uint64_t m0 = lo + (uint64_t)(lane + 1) * step - 1, m1 = m0 + 32 * step;
+    const bool in0 = m0 < hi, in1 = m1 < hi;
+    K a0 = K(), b0 = K(), a1 = K(), b1 = K();
+    if (in0) {
+      a0 = a[m0];
+      b0 = b[diag - 1 - m0];
+    }
+    if (in1) {
+      a1 = a[m1];
+      b1 = b[diag - 1 - m1];
+    }
+    const unsigned int s0 = __ballot_sync(0xffffffffu, !in0 || b0 < a0), s1 = __ballot_sync(0xffffffffu, !in1 || b1 < a1);
+    const unsigned int f = s0 ? (unsigned int)__ffs(s0) - 1u : s1 ? (unsigned int)__ffs(s1) + 31u : 64u;  // first probe past the split
+    if (f < 64u && lo + (uint64_t)(f + 1) * step - 1 < hi) hi = lo + (uint64_t)(f + 1) * step - 1;
+    lo += (uint64_t)f * step;
+  }
+  return hi;
+}
+
 // What the compute warps need to know of a tile in a buffer (written by the
 // loader before it arms the buffer's barrier).
 struct MergeDesc {
@@ -75,6 +106,7 @@ struct MergeDesc {
   uint32_t ia, ib;    // index of A's / B's first element in the keys (and payloads) area
   uint32_t count;     // outputs (la + lb)
   uint32_t tile;      // tile index
+  uint64_t a0;        // A's first element of the tile
 };
 
 // The kernel's parameters.
@@ -90,7 +122,7 @@ struct MergeArgs {
   uint64_t nb;
   K *out;
   P *outv;
-  const uint64_t *parts;
+  const uint64_t *parts;  // the split at every tile boundary, or null: the loader warp finds them
   uint64_t tiles;
   uint64_t covered_out;  // leading outputs inside whole rows of both output views (0: none)
   int tma_in;            // a, b, av, bv 16-byte aligned: inputs arrive by bulk copies
@@ -118,8 +150,15 @@ __device__ __forceinline__ void merge_load_range(T *dst, const T *src, uint64_t 
 }
 
 // Persistent merge.  Warps 0-7 merge; warp 8's lane 0 loads and stores.
-// CTA c takes tiles c, c + G, c + 2G, ... (G = gridDim.x); tile i of the CTA
-// uses buffer i mod 2 and goes through:
+// CTA c takes the c-th of gridDim.x equal runs of consecutive tiles.  Where a
+// tile's inputs begin (its split) comes from a partition kernel or, with few
+// tiles a CTA, from the loader warp itself, two tiles ahead: a tile's split
+// lies within a tile of the one before, so its search reads what is loaded
+// next anyway and runs while the compute warps merge.  (The partition kernel,
+// one thread a split, waits for 21 to 26 reads one after another: 14 us before
+// a merge of 3.7 million i32 keys that takes 12.)  A warp of its own for the
+// searches made the kernel's registers spill: 447 us for 2 x 2^26 f32/u32
+// pairs against 408.  Tile i of the CTA uses buffer i mod 2 and goes through:
 //   loader: (once the compute warps have written tile i-2's outputs to the
 //           buffer and that tile's stores have read them) write the tile's
 //           descriptor, bulk-copy its ranges in; full[b] completes;
@@ -160,12 +199,47 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
   }
   __syncthreads();
 
-  // tiles of this CTA: blockIdx.x + i * G for i < mine (the grid is no larger than the tile count)
-  const uint64_t mine = (args.tiles - blockIdx.x + G - 1) / G;
+  // tiles of this CTA: first + i for i < mine (the grid is no larger than the tile count)
+  const uint64_t first = args.tiles * blockIdx.x / G, mine = args.tiles * (blockIdx.x + 1) / G - first;
 
   if (warp == kMergeWarps) {
-    // ================= the loader (lane 0) =================
-    if (lane != 0) return;
+    // ================= the loader (lane 0; the splits: all lanes) =================
+    // A elements before tile k, given that `from` lie before a tile no more than `tiles` before it
+    auto split = [&](uint64_t k, uint64_t from, uint64_t tiles) -> uint64_t {
+      const uint64_t diag = k * TILE < total ? k * TILE : total;
+      uint64_t lo = diag > args.nb ? diag - args.nb : 0, hi = diag < args.na ? diag : args.na;
+      if (lo < from) lo = from;
+      if (hi > from + tiles * TILE) hi = from + tiles * TILE;
+      return merge_split_warp(args.a, args.b, diag, lo, hi, lane);
+    };
+    // Into L2: tile k's payloads (its A range [f, t)) and the keys that the
+    // search for the tile after it can reach.
+    uint64_t pa = 0, pb = 0;  // keys up to here have been asked for
+    auto prefetch = [&](uint64_t k, uint64_t f, uint64_t t) {
+      const uint64_t d0 = k * TILE, d1 = d0 + TILE < total ? d0 + TILE : total;
+      if constexpr (HP) {
+        prefetch_l2_range(args.av + f, (t - f) * sizeof(P));
+        prefetch_l2_range(args.bv + (d0 - f), (d1 - d0 - (t - f)) * sizeof(P));
+      }
+      const uint64_t ea = t + TILE < args.na ? t + TILE : args.na;
+      const uint64_t eb = d1 - t + TILE < args.nb ? d1 - t + TILE : args.nb;
+      if (pa < f) pa = f;
+      if (pb < d0 - f) pb = d0 - f;
+      if (pa < ea) prefetch_l2_range(args.a + pa, (ea - pa) * sizeof(K));
+      if (pb < eb) prefetch_l2_range(args.b + pb, (eb - pb) * sizeof(K));
+      pa = ea;
+      pb = eb;
+    };
+    const uint64_t *const parts = args.parts;
+    uint64_t a0, a1;  // the A range of the tile to load next
+    if (parts != nullptr) {
+      a0 = parts[first];
+      a1 = parts[first + 1];
+    } else {
+      a0 = split(first, 0, first);
+      a1 = split(first + 1, a0, 1);
+      if (lane == 0 && mine > 1) prefetch(first, a0, a1);
+    }
     const uint64_t policy = l2_policy_evict_first();  // inputs and outputs are read / written once
     uint32_t outpar = 0u, armpar = 0u, armany = 0u;
     bool stored = false, failed = false;
@@ -174,14 +248,14 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
       const int b = (int)(i & 1);
       if (i >= 2) {
         // tile i-2's outputs are in buffer b: store them
-        if (!mbar_wait_or_abort(&s_out[b], (outpar >> b) & 1u, spin_limit_ns, &s_abort)) {
+        if (lane == 0 && !mbar_wait_or_abort(&s_out[b], (outpar >> b) & 1u, spin_limit_ns, &s_abort)) {
           failed = true;
-          fail_tile = blockIdx.x + (i - 2) * G;
-          break;
+          fail_tile = first + i - 2;
         }
+        if (__shfl_sync(0xffffffffu, (int)failed, 0)) break;
         outpar ^= 1u << b;
         const uint32_t tile = s_desc[b].tile;
-        if (args.covered_out > (uint64_t)tile * TILE) {
+        if (lane == 0 && args.covered_out > (uint64_t)tile * TILE) {
           tma_store_rows(&args.okmap, tile * C::KROWS, buf(b), policy);
           if constexpr (HP) tma_store_rows(&args.opmap, tile * C::PROWS, buf(b) + C::KEY_AREA, policy);
           tma_store_commit();
@@ -189,45 +263,59 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
         }
       }
       if (i >= mine) continue;
-      if (stored) tma_store_wait_read();  // the stores have read the buffer
       // ---- tile k: its A range [a0, a1) and B range [b0, b1)
-      const uint64_t k = blockIdx.x + i * G;
-      const uint64_t d0 = k * TILE, d1 = d0 + TILE < total ? d0 + TILE : total;
-      const uint64_t a0 = args.parts[k], a1 = args.parts[k + 1];
-      const uint64_t b0 = d0 - a0, b1 = d1 - a1;
-      MergeDesc d;
-      d.la = (uint32_t)(a1 - a0);
-      d.lb = (uint32_t)(b1 - b0);
-      d.count = (uint32_t)(d1 - d0);
-      d.tile = (uint32_t)k;
-      if (args.tma_in) {
-        const uint64_t alo = a0 & ~(uint64_t)(C::L - 1), blo = b0 & ~(uint64_t)(C::L - 1);
-        const uint32_t bstart = (uint32_t)align_up(a1 - alo, (size_t)C::L);  // B's copy: a multiple of L
-        d.ia = (uint32_t)(a0 - alo);
-        d.ib = bstart + (uint32_t)(b0 - blo);
-        uint32_t bytes = (a1 > a0 ? merge_bulk_bytes<K>(alo, a1) : 0u) + (b1 > b0 ? merge_bulk_bytes<K>(blo, b1) : 0u);
-        if constexpr (HP)
-          bytes += (a1 > a0 ? merge_bulk_bytes<P>(alo, a1) : 0u) + (b1 > b0 ? merge_bulk_bytes<P>(blo, b1) : 0u);
-        if (bytes) mbar_expect_tx(&s_full[b], bytes);
-        K *sk = reinterpret_cast<K *>(buf(b));
-        P *sp = reinterpret_cast<P *>(buf(b) + C::KEY_AREA);
-        if (a1 > a0) merge_load_range<K>(sk, args.a, alo, a1, &s_full[b], policy);
-        if (b1 > b0) merge_load_range<K>(sk + bstart, args.b, blo, b1, &s_full[b], policy);
-        if constexpr (HP) {
-          if (a1 > a0) merge_load_range<P>(sp, args.av, alo, a1, &s_full[b], policy);
-          if (b1 > b0) merge_load_range<P>(sp + bstart, args.bv, blo, b1, &s_full[b], policy);
+      const uint64_t k = first + i;
+      if (lane == 0) {
+        if (stored) tma_store_wait_read();  // the stores have read the buffer
+        const uint64_t d0 = k * TILE, d1 = d0 + TILE < total ? d0 + TILE : total;
+        const uint64_t b0 = d0 - a0, b1 = d1 - a1;
+        MergeDesc d;
+        d.la = (uint32_t)(a1 - a0);
+        d.lb = (uint32_t)(b1 - b0);
+        d.count = (uint32_t)(d1 - d0);
+        d.tile = (uint32_t)k;
+        d.a0 = a0;
+        if (args.tma_in) {
+          const uint64_t alo = a0 & ~(uint64_t)(C::L - 1), blo = b0 & ~(uint64_t)(C::L - 1);
+          const uint32_t bstart = (uint32_t)align_up(a1 - alo, (size_t)C::L);  // B's copy: a multiple of L
+          d.ia = (uint32_t)(a0 - alo);
+          d.ib = bstart + (uint32_t)(b0 - blo);
+          uint32_t bytes =
+              (a1 > a0 ? merge_bulk_bytes<K>(alo, a1) : 0u) + (b1 > b0 ? merge_bulk_bytes<K>(blo, b1) : 0u);
+          if constexpr (HP)
+            bytes += (a1 > a0 ? merge_bulk_bytes<P>(alo, a1) : 0u) + (b1 > b0 ? merge_bulk_bytes<P>(blo, b1) : 0u);
+          if (bytes) mbar_expect_tx(&s_full[b], bytes);
+          K *sk = reinterpret_cast<K *>(buf(b));
+          P *sp = reinterpret_cast<P *>(buf(b) + C::KEY_AREA);
+          if (a1 > a0) merge_load_range<K>(sk, args.a, alo, a1, &s_full[b], policy);
+          if (b1 > b0) merge_load_range<K>(sk + bstart, args.b, blo, b1, &s_full[b], policy);
+          if constexpr (HP) {
+            if (a1 > a0) merge_load_range<P>(sp, args.av, alo, a1, &s_full[b], policy);
+            if (b1 > b0) merge_load_range<P>(sp + bstart, args.bv, blo, b1, &s_full[b], policy);
+          }
+        } else {  // the compute warps copy the ranges themselves
+          d.ia = 0;
+          d.ib = d.la;
         }
-      } else {  // the compute warps copy the ranges themselves
-        d.ia = 0;
-        d.ib = d.la;
+        s_desc[b] = d;
+        // the loader's one arrival, after its plain stores (descriptor, ragged
+        // ends): the phase completes once the bulk copies' bytes have landed
+        mbar_arrive(&s_full[b]);
       }
-      s_desc[b] = d;
-      // the loader's one arrival, after its plain stores (descriptor, ragged
-      // ends): the phase completes once the bulk copies' bytes have landed
-      mbar_arrive(&s_full[b]);
+      __syncwarp();
       armpar ^= 1u << b;
       armany |= 1u << b;
+      if (i + 1 < mine) {  // the next tile's end, while this one is merged
+        a0 = a1;
+        if (parts != nullptr) {
+          a1 = parts[k + 2];
+        } else {
+          a1 = split(k + 2, a0, 1);
+          if (lane == 0) prefetch(k + 1, a0, a1);
+        }
+      }
     }
+    if (lane != 0) return;
     if (failed) {
       record_error(hdr, BK_ERR_SPIN_TIMEOUT, (unsigned int)fail_tile);
       *reinterpret_cast<volatile int *>(&s_abort) = 1;
@@ -244,7 +332,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
   bool bad = false;
   for (uint64_t i = 0; i < mine; ++i) {
     const int b = (int)(i & 1);
-    const uint64_t k = blockIdx.x + i * G;
+    const uint64_t k = first + i;
     if (!mbar_wait_or_abort(&s_full[b], (fullpar >> b) & 1u, spin_limit_ns, &s_abort)) bad = true;
     fullpar ^= 1u << b;
     if (named_barrier_or(1, kMergeCompute, bad || aborted())) {
@@ -256,7 +344,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     K *const sk = reinterpret_cast<K *>(buf(b));
     P *const sp = reinterpret_cast<P *>(buf(b) + C::KEY_AREA);
     if (!args.tma_in) {  // a launch-wide flag: every compute warp takes this branch or none
-      const uint64_t d0 = k * TILE, a0 = args.parts[k], b0 = d0 - a0;
+      const uint64_t a0 = d.a0, b0 = k * TILE - a0;
       for (uint32_t j = tid; j < d.la; j += kMergeCompute) {
         sk[j] = args.a[a0 + j];
         if constexpr (HP) sp[j] = args.av[a0 + j];
@@ -270,7 +358,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     // ---- merge-path search for this thread's first output, then its outputs
     const uint32_t diag = (uint32_t)tid * ITEMS;
     K okey[ITEMS];
-    uint32_t osrc[ITEMS];
+    uint32_t osrc[ITEMS / 2];  // indexes of the outputs' sources, two to a register
     const int valid = (int)min((int)d.count - (int)diag, ITEMS);
     if (valid > 0) {
       uint32_t lo = diag > d.lb ? diag - d.lb : 0u;
@@ -291,7 +379,9 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
           // take A while B is exhausted or !(b < a): equal keys keep A first
           const bool take_a = ia < ea && (ib >= eb || !(kb < ka));
           okey[j] = take_a ? ka : kb;
-          osrc[j] = take_a ? ia : ib;
+          const uint32_t at = take_a ? ia : ib;
+          if (j & 1) osrc[j >> 1] |= at << 16;
+          else osrc[j >> 1] = at;
           ia += take_a ? 1u : 0u;
           ib += take_a ? 0u : 1u;
           if (j + 1 < ITEMS) {
@@ -306,7 +396,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     if constexpr (HP) {
 #pragma unroll
       for (int j = 0; j < ITEMS; ++j)
-        if (j < valid) opay[j] = sp[osrc[j]];
+        if (j < valid) opay[j] = sp[(j & 1) ? osrc[j >> 1] >> 16 : osrc[j >> 1] & 0xffffu];
     }
     named_barrier_sync(2, kMergeCompute);  // every thread has read its inputs
     // ---- outputs: in place, swizzled for the tensor stores (which write
@@ -383,10 +473,6 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   st = host::check_ws(d_ws, ws_bytes, merge_ws_bytes<K>(n));
   if (st != BK_OK) return st;
   WsHeader *hdr = reinterpret_cast<WsHeader *>(d_ws);
-  uint64_t *parts = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(d_ws) + kHeaderBytes);
-  const uint64_t np = tiles + 1;
-  merge_partition_kernel<K><<<(unsigned)((np + 255) / 256), 256, 0, stream>>>(a, na, b, nb, C::TILE, np, parts);
-  if ((st = host::launch_status()) != BK_OK) return st;
 
   MergeArgs<K, P> args;
   memset(&args, 0, sizeof(args));
@@ -398,7 +484,6 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   args.nb = nb;
   args.out = out;
   args.outv = outv;
-  args.parts = parts;
   args.tiles = tiles;
   auto a16 = [](const void *p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   args.tma_in = a16(a) && a16(b) && a16(av) && a16(bv);
@@ -422,6 +507,21 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   const uint64_t per_sm = ks.resident_ctas / (uint64_t)di.sm_count;  // what fits (shared memory, registers)
   const uint64_t want = (uint64_t)di.sm_count * (uint64_t)std::max(kn.ctas_per_sm, 1);
   const unsigned grid = (unsigned)std::min<uint64_t>(tiles, std::min<uint64_t>(want, std::max<uint64_t>(per_sm, 1) * di.sm_count));
+  // Many tiles a CTA: a partition kernel first, whose splits cost the loader
+  // nothing; few: the loader finds them (see merge_kernel).  Measured on a
+  // B200, partition / loader: f32/u32 2 x 2^18 17.4 / 13.0 us, 2 x 2^22 46.1 /
+  // 37.9, 2 x 2^24 (18 tiles a CTA) 113.7 / 113.6, 2 x 2^25 201.7 / 206.8;
+  // f64/u32 2 x 2^21 39.8 / 33.6, 2 x 2^22 (9 a CTA) 62.5 / 62.3, 2 x 2^24
+  // 169 / 181; f64 2 x 2^22 52.2 / 47.1, 2 x 2^24 136.2 / 135.2; f32 2 x 2^18
+  // 15.3 / 11.1, 2 x 2^26 273 / 262 (keys of 4 bytes alone never need it).
+  constexpr uint64_t kPerCta = C::PB == 0 ? (sizeof(K) == 4 ? ~0ull : 16) : (sizeof(K) == 4 ? 16 : 8);
+  if (tiles / kPerCta >= grid) {
+    uint64_t *parts = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(d_ws) + kHeaderBytes);
+    const uint64_t np = tiles + 1;
+    merge_partition_kernel<K><<<(unsigned)((np + 255) / 256), 256, 0, stream>>>(a, na, b, nb, C::TILE, np, parts);
+    if ((st = host::launch_status()) != BK_OK) return st;
+    args.parts = parts;
+  }
   const host::DebugFault dbg = host::debug_fault();
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
   merge_kernel<K, P><<<grid, kMergeThreads, smem, stream>>>(args, hdr, limit);

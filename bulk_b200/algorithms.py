@@ -24,8 +24,8 @@ libbulkb200.so.  Errors raise :class:`bulk_b200.BulkError`.
 """
 from __future__ import annotations
 
-import ctypes
 import threading
+from functools import lru_cache
 
 import torch
 
@@ -50,20 +50,22 @@ def dtype_tag(t: torch.dtype) -> str:
         raise TypeError(f"unsupported dtype {t}") from None
 
 
-def _ptr(t: torch.Tensor | None) -> int | None:
-    return None if t is None else t.data_ptr()
-
-
 def _stream_obj(stream: torch.cuda.Stream | None, device: torch.device) -> torch.cuda.Stream:
     return stream if stream is not None else torch.cuda.current_stream(device)
 
 
+# the current stream's raw handle without a Stream object around it, where torch has it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_handle(stream: torch.cuda.Stream | None, device: torch.device) -> int:
+    if stream is None and _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
     return _stream_obj(stream, device).cuda_stream
 
 
 def _require_cuda(*ts: torch.Tensor) -> torch.device:
-    dev = None
+    first = None
     for t in ts:
         if t is None:
             continue
@@ -71,11 +73,11 @@ def _require_cuda(*ts: torch.Tensor) -> torch.device:
             raise ValueError("bulk_b200 operates on CUDA tensors (device memory)")
         if not t.is_contiguous():
             raise ValueError("bulk_b200 needs contiguous tensors")
-        if dev is None:
-            dev = t.device
-        elif t.device != dev:
+        if first is None:
+            first, index = t, t.get_device()
+        elif t.get_device() != index:
             raise ValueError("all tensors must be on the same device")
-    return dev
+    return None if first is None else first.device
 
 
 class _WorkspacePool:
@@ -92,27 +94,32 @@ class _WorkspacePool:
 
     def __init__(self):
         self._lock = threading.Lock()
-        self._ws: dict[tuple[int, int], torch.Tensor] = {}
+        self._ws: dict[tuple[int, int], tuple[torch.Tensor, int, int]] = {}  # the buffer, its address and size
 
-    def get(self, nbytes: int, device: torch.device, stream: torch.cuda.Stream) -> tuple[int, int]:
-        key = (device.index if device.index is not None else torch.cuda.current_device(), stream.cuda_stream)
+    def get(self, nbytes: int, device: torch.device, stream: torch.cuda.Stream | None,
+            handle: int | None = None) -> tuple[int, int]:
+        """(pointer, bytes) of the workspace of ``stream`` (``handle``: its
+        raw handle, when the caller has it; None: the current stream)."""
+        if handle is None:
+            handle = _stream_handle(stream, device)
+        key = (device.index if device.index is not None else torch.cuda.current_device(), handle)
         with self._lock:
-            t = self._ws.get(key)
-            if t is None or t.numel() < nbytes:
-                size = max(nbytes, 1 << 16, 0 if t is None else 2 * t.numel())
-                with torch.cuda.stream(stream):
+            have = self._ws.get(key)
+            if have is None or have[2] < nbytes:
+                size = max(nbytes, 1 << 16, 0 if have is None else 2 * have[2])
+                with torch.cuda.stream(_stream_obj(stream, device)):
                     t = torch.zeros(size, dtype=torch.uint8, device=device)
-                self._ws[key] = t
-            return t.data_ptr(), t.numel()
+                have = self._ws[key] = (t, t.data_ptr(), size)
+            return have[1], have[2]
 
     def status(self, device: torch.device | None = None, stream: torch.cuda.Stream | None = None) -> int:
         device = device or torch.device("cuda", torch.cuda.current_device())
         s = _stream_handle(stream, device)
         key = (device.index if device.index is not None else torch.cuda.current_device(), s)
-        t = self._ws.get(key)
-        if t is None:
+        have = self._ws.get(key)
+        if have is None:
             return _lib.BK_OK
-        return lib.bk_workspace_status(t.data_ptr(), t.numel(), s)
+        return lib.bk_workspace_status(have[1], have[2], s)
 
     def clear(self):
         with self._lock:
@@ -135,11 +142,32 @@ def debug_set_fault(skip_publish_tile: int = -1, spin_limit_ns: int = 0) -> None
     check(lib.bk_debug_set_fault(skip_publish_tile, spin_limit_ns), "bk_debug_set_fault")
 
 
-def _ws(algo, key, value, n, device, stream: torch.cuda.Stream):
-    need = workspace_bytes(algo, key, value, n)
-    if need == 0 and algo not in ("reduce",):
-        return None, 0
-    return workspaces.get(max(need, 256), device, stream)
+# The workspace a call needs depends on its types and length alone: kept for
+# the lengths in use, so that a repeated call asks the library once.
+_need_bytes = lru_cache(maxsize=4096)(workspace_bytes)
+
+
+@lru_cache(maxsize=None)
+def _entry(*name: str):
+    """The library's entry point bk_<name parts joined>."""
+    return getattr(lib, "bk_" + "_".join(name))
+
+
+def _call(fn, dev: torch.device, stream: torch.cuda.Stream | None, need: int, *args) -> None:
+    """``fn(*args, workspace, its bytes, stream)`` with ``dev`` current; no workspace where ``need`` is 0."""
+    if dev.index != torch.cuda.current_device():
+        with torch.cuda.device(dev):
+            return _call(fn, dev, stream, need, *args)
+    s = _stream_handle(stream, dev)
+    ws, wsb = workspaces.get(need, dev, stream, s) if need else (None, 0)
+    status = fn(*args, ws, wsb, s)
+    if status != _lib.BK_OK:
+        check(status, fn.__name__)
+
+
+def _need(algo: str, key: str, value: str | None, n: int) -> int:
+    need = _need_bytes(algo, key, value, n)
+    return max(need, 256) if need or algo == "reduce" else 0
 
 
 # ---------------------------------------------------------------------------
@@ -150,12 +178,8 @@ def reduce(x: torch.Tensor, init=0, op: str = "sum", out: torch.Tensor | None = 
     tag = dtype_tag(x.dtype)
     if out is None:
         out = torch.empty(1, dtype=x.dtype, device=dev)
-    with torch.cuda.device(dev):
-        so = _stream_obj(stream, dev)
-        s = so.cuda_stream
-        ws, wsb = _ws("reduce", tag, None, x.numel(), dev, so)
-        fn = getattr(lib, f"bk_reduce_{op}_{tag}")
-        check(fn(_ptr(x), x.numel(), init, _ptr(out), ws, wsb, s), fn.__name__)
+    n = x.numel()
+    _call(_entry("reduce", op, tag), dev, stream, _need("reduce", tag, None, n), x.data_ptr(), n, init, out.data_ptr())
     return out
 
 
@@ -174,16 +198,13 @@ def inclusive_scan(x: torch.Tensor, init=0, op: str = "sum", out: torch.Tensor |
     if dinit:
         if not init.is_cuda or init.device != dev or init.dtype != x.dtype or init.numel() != 1:
             raise ValueError("a tensor init must be one element of x's dtype on x's device")
-    with torch.cuda.device(dev):
-        so = _stream_obj(stream, dev)
-        s = so.cuda_stream
-        ws, wsb = _ws("inclusive_scan", tag, None, x.numel(), dev, so)
-        if dinit:
-            fn = getattr(lib, f"bk_inclusive_scan_{op}_{tag}_dinit")
-            check(fn(_ptr(x), x.numel(), _ptr(init), _ptr(out), ws, wsb, s), fn.__name__)
-        else:
-            fn = getattr(lib, f"bk_inclusive_scan_{op}_{tag}")
-            check(fn(_ptr(x), x.numel(), init, _ptr(out), ws, wsb, s), fn.__name__)
+    n = x.numel()
+    need = _need("inclusive_scan", tag, None, n)
+    if dinit:
+        _call(_entry("inclusive_scan", op, tag, "dinit"), dev, stream, need, x.data_ptr(), n, init.data_ptr(),
+              out.data_ptr())
+    else:
+        _call(_entry("inclusive_scan", op, tag), dev, stream, need, x.data_ptr(), n, init, out.data_ptr())
     return out
 
 
@@ -212,17 +233,13 @@ def merge(a: torch.Tensor, b: torch.Tensor, a_vals: torch.Tensor | None = None, 
         raise TypeError("a_vals and b_vals must both be given, with the same element size")
     if a_vals is not None and out_vals is None:
         out_vals = torch.empty(n, dtype=a_vals.dtype, device=dev)
-    with torch.cuda.device(dev):
-        so = _stream_obj(stream, dev)
-        s = so.cuda_stream
-        ws, wsb = _ws("merge", tag, _payload_tag(a_vals), n, dev, so)
-        if a_vals is None:
-            fn = getattr(lib, f"bk_merge_{tag}")
-            check(fn(_ptr(a), a.numel(), _ptr(b), b.numel(), _ptr(out), ws, wsb, s), fn.__name__)
-            return out
-        fn = getattr(lib, f"bk_merge_by_key_{tag}_{_payload_tag(a_vals)}")
-        check(fn(_ptr(a), _ptr(a_vals), a.numel(), _ptr(b), _ptr(b_vals), b.numel(), _ptr(out), _ptr(out_vals),
-                 ws, wsb, s), fn.__name__)
+    vt = _payload_tag(a_vals)
+    need = _need("merge", tag, vt, n)
+    if a_vals is None:
+        _call(_entry("merge", tag), dev, stream, need, a.data_ptr(), a.numel(), b.data_ptr(), b.numel(), out.data_ptr())
+        return out
+    _call(_entry("merge_by_key", tag, vt), dev, stream, need, a.data_ptr(), a_vals.data_ptr(), a.numel(), b.data_ptr(),
+          b_vals.data_ptr(), b.numel(), out.data_ptr(), out_vals.data_ptr())
     return out, out_vals
 
 
@@ -234,16 +251,12 @@ def stable_sort_by_key(keys: torch.Tensor, vals: torch.Tensor | None = None,
     n = keys.numel()
     if vals is not None and vals.numel() != n:
         raise ValueError("keys and vals must have the same length")
-    with torch.cuda.device(dev):
-        so = _stream_obj(stream, dev)
-        s = so.cuda_stream
-        ws, wsb = _ws("sort_by_key", tag, _payload_tag(vals), n, dev, so)
-        if vals is None:
-            fn = getattr(lib, f"bk_sort_keys_{tag}")
-            check(fn(_ptr(keys), n, ws, wsb, s), fn.__name__)
-            return keys
-        fn = getattr(lib, f"bk_sort_by_key_{tag}_{_payload_tag(vals)}")
-        check(fn(_ptr(keys), _ptr(vals), n, ws, wsb, s), fn.__name__)
+    vt = _payload_tag(vals)
+    need = _need("sort_by_key", tag, vt, n)
+    if vals is None:
+        _call(_entry("sort_keys", tag), dev, stream, need, keys.data_ptr(), n)
+        return keys
+    _call(_entry("sort_by_key", tag, vt), dev, stream, need, keys.data_ptr(), vals.data_ptr(), n)
     return keys, vals
 
 
@@ -268,13 +281,8 @@ def reduce_by_key(keys: torch.Tensor, vals: torch.Tensor, out_keys: torch.Tensor
         out_vals = torch.empty(max(n, 1), dtype=vals.dtype, device=dev)
     if num_out is None:
         num_out = torch.empty(1, dtype=torch.int64, device=dev)
-    with torch.cuda.device(dev):
-        so = _stream_obj(stream, dev)
-        s = so.cuda_stream
-        ws, wsb = _ws("reduce_by_key", kt, vt, n, dev, so)
-        fn = getattr(lib, f"bk_reduce_by_key_{kt}_{vt}")
-        check(fn(_ptr(keys), _ptr(vals), n, _ptr(out_keys), _ptr(out_vals), _ptr(num_out), ws, wsb, s),
-              fn.__name__)
+    _call(_entry("reduce_by_key", kt, vt), dev, stream, _need("reduce_by_key", kt, vt, n), keys.data_ptr(),
+          vals.data_ptr(), n, out_keys.data_ptr(), out_vals.data_ptr(), num_out.data_ptr())
     if not sync:
         return out_keys, out_vals, num_out
     c = int(num_out.item())

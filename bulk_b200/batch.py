@@ -12,13 +12,15 @@ libbulkb200.so.  Errors raise :class:`bulk_b200.BulkError`.
 from __future__ import annotations
 
 import ctypes
+import operator
+import struct
 from functools import lru_cache
 
 import torch
 
 from . import _lib
-from ._lib import check, lib
-from .algorithms import _require_cuda, _stream_obj, dtype_tag, workspaces
+from ._lib import lib
+from .algorithms import _call, _entry, _require_cuda, dtype_tag
 
 BATCH_MAX = 256
 
@@ -63,6 +65,26 @@ def batch_workspace_bytes(algo: str, key: str, value: str | None, sizes) -> int:
     return lib.bk_batch_workspace_bytes(_lib.ALGO[algo], _lib.DTYPE[key], _lib.DTYPE[value], arr, len(sizes))
 
 
+# struct codes of the items' fields (pointers and lengths are 64-bit; an init
+# value narrower than that is followed by its struct's tail padding).  Init
+# values are converted as a C assignment converts them: integers mod 2^32 or
+# 2^64, floats too large for f32 to infinity.
+_INIT_CODE = {"i32": "I4x", "u32": "I4x", "i64": "Q", "u64": "Q", "f32": "f4x", "f64": "d"}
+
+
+def _init_value(tag: str, init):
+    if tag in ("f32", "f64"):
+        return _CT[tag](init).value
+    return operator.index(init) & (0xFFFFFFFF if tag in ("i32", "u32") else 0xFFFFFFFFFFFFFFFF)
+
+
+def _issue(fn, dev, stream, algo: str, kt: str, vt: str | None, sizes, code: str, rows) -> None:
+    """One batched call of ``rows`` (the items' fields in order, ``code`` each), packed in one go."""
+    items = struct.pack("=" + code * len(rows), *[f for row in rows for f in row])
+    need = max(batch_workspace_bytes(algo, kt, vt, sizes), 256)
+    _call(fn, dev, stream, need, items, len(rows))
+
+
 def _chunks(n: int):
     for lo in range(0, n, BATCH_MAX):
         yield lo, min(n, lo + BATCH_MAX)
@@ -82,19 +104,11 @@ def inclusive_scan_batch(xs, inits=None, outs=None, stream: torch.cuda.Stream | 
     outs = list(outs) if outs is not None else [torch.empty_like(x) for x in xs]
     if len(inits) != len(xs) or len(outs) != len(xs):
         raise ValueError("xs, inits and outs must have the same length")
-    so = _stream_obj(stream, dev)
-    s = so.cuda_stream
-    item_t = scan_item_type(tag)
-    fn = getattr(lib, f"bk_inclusive_scan_sum_{tag}_batch")
+    fn = _entry("inclusive_scan_sum", tag, "batch")
+    sizes = [x.numel() for x in xs]
+    rows = [(x.data_ptr(), o.data_ptr(), n, _init_value(tag, i)) for x, o, n, i in zip(xs, outs, sizes, inits)]
     for lo, hi in _chunks(len(xs)):
-        items = (item_t * (hi - lo))()
-        for j, k in enumerate(range(lo, hi)):
-            items[j].d_in, items[j].d_out, items[j].n, items[j].init = xs[k].data_ptr(), outs[k].data_ptr(), \
-                xs[k].numel(), inits[k]
-        need = batch_workspace_bytes("inclusive_scan", tag, None, [xs[k].numel() for k in range(lo, hi)])
-        with torch.cuda.device(dev):
-            ws, wsb = workspaces.get(max(need, 256), dev, so)
-            check(fn(ctypes.cast(items, ctypes.c_void_p), hi - lo, ws, wsb, s), fn.__name__)
+        _issue(fn, dev, stream, "inclusive_scan", tag, None, sizes[lo:hi], "3Q" + _INIT_CODE[tag], rows[lo:hi])
     return outs
 
 
@@ -119,10 +133,7 @@ def reduce_by_key_batch(keys_list, vals_list, stream: torch.cuda.Stream | None =
             raise TypeError("one key dtype and one value dtype per batch")
         if k.numel() != v.numel():
             raise ValueError("keys and vals must have the same length")
-    so = _stream_obj(stream, dev)
-    s = so.cuda_stream
-    item_t = rbk_item_type(kt, vt)
-    fn = getattr(lib, f"bk_reduce_by_key_{kt}_{vt}_batch")
+    fn = _entry("reduce_by_key", kt, vt, "batch")
     if outs is not None:
         outs = list(outs)
         if len(outs) != len(keys_list):
@@ -137,17 +148,11 @@ def reduce_by_key_batch(keys_list, vals_list, stream: torch.cuda.Stream | None =
             res.append((torch.empty(max(k.numel(), 1), dtype=k.dtype, device=dev),
                         torch.empty(max(v.numel(), 1), dtype=v.dtype, device=dev)))
         cnt = [counts[i:i + 1] for i in range(len(keys_list))]
-    for lo, hi in _chunks(len(keys_list)):
-        items = (item_t * (hi - lo))()
-        for j, i in enumerate(range(lo, hi)):
-            it = items[j]
-            it.keys, it.vals, it.n = keys_list[i].data_ptr(), vals_list[i].data_ptr(), keys_list[i].numel()
-            it.out_keys, it.out_vals = res[i][0].data_ptr(), res[i][1].data_ptr()
-            it.d_num_out = cnt[i].data_ptr()
-        need = batch_workspace_bytes("reduce_by_key", kt, vt, [keys_list[i].numel() for i in range(lo, hi)])
-        with torch.cuda.device(dev):
-            ws, wsb = workspaces.get(max(need, 256), dev, so)
-            check(fn(ctypes.cast(items, ctypes.c_void_p), hi - lo, ws, wsb, s), fn.__name__)
+    sizes = [k.numel() for k in keys_list]
+    rows = [(k.data_ptr(), v.data_ptr(), n, r[0].data_ptr(), r[1].data_ptr(), c.data_ptr())
+            for k, v, n, r, c in zip(keys_list, vals_list, sizes, res, cnt)]
+    for lo, hi in _chunks(len(rows)):
+        _issue(fn, dev, stream, "reduce_by_key", kt, vt, sizes[lo:hi], "6Q", rows[lo:hi])
     if not sync:
         return [(ok, ov, cnt[i]) for i, (ok, ov) in enumerate(res)]
     cs = [int(c) for c in torch.cat([c.view(1) for c in cnt]).tolist()]
@@ -173,19 +178,11 @@ def stable_sort_by_key_batch(keys_list, vals_list, stream: torch.cuda.Stream | N
             raise TypeError("one key dtype and one payload size per batch")
         if k.numel() != v.numel():
             raise ValueError("keys and vals must have the same length")
-    so = _stream_obj(stream, dev)
-    s = so.cuda_stream
-    item_t = sort_item_type(kt, vt)
-    fn = getattr(lib, f"bk_sort_by_key_{kt}_{vt}_batch")
-    for lo, hi in _chunks(len(keys_list)):
-        items = (item_t * (hi - lo))()
-        for j, i in enumerate(range(lo, hi)):
-            items[j].keys, items[j].vals, items[j].n = keys_list[i].data_ptr(), vals_list[i].data_ptr(), \
-                keys_list[i].numel()
-        need = batch_workspace_bytes("sort_by_key", kt, vt, [keys_list[i].numel() for i in range(lo, hi)])
-        with torch.cuda.device(dev):
-            ws, wsb = workspaces.get(max(need, 256), dev, so)
-            check(fn(ctypes.cast(items, ctypes.c_void_p), hi - lo, ws, wsb, s), fn.__name__)
+    fn = _entry("sort_by_key", kt, vt, "batch")
+    sizes = [k.numel() for k in keys_list]
+    rows = [(k.data_ptr(), v.data_ptr(), n) for k, v, n in zip(keys_list, vals_list, sizes)]
+    for lo, hi in _chunks(len(rows)):
+        _issue(fn, dev, stream, "sort_by_key", kt, vt, sizes[lo:hi], "3Q", rows[lo:hi])
     return keys_list, vals_list
 
 
@@ -213,18 +210,10 @@ def stable_sort_by_key_copy_batch(in_keys, in_vals, out_keys=None, out_vals=None
             raise TypeError("one key dtype and one payload size per batch")
         if not (k.numel() == v.numel() == ok.numel() == ov.numel()):
             raise ValueError("every array of an item must have the same length")
-    so = _stream_obj(stream, dev)
-    s = so.cuda_stream
-    item_t = sort_copy_item_type(kt, vt)
-    fn = getattr(lib, f"bk_sort_by_key_{kt}_{vt}_copy_batch")
-    for lo, hi in _chunks(len(in_keys)):
-        items = (item_t * (hi - lo))()
-        for j, i in enumerate(range(lo, hi)):
-            it = items[j]
-            it.in_keys, it.in_vals = in_keys[i].data_ptr(), in_vals[i].data_ptr()
-            it.keys, it.vals, it.n = out_keys[i].data_ptr(), out_vals[i].data_ptr(), in_keys[i].numel()
-        need = batch_workspace_bytes("sort_by_key", kt, vt, [in_keys[i].numel() for i in range(lo, hi)])
-        with torch.cuda.device(dev):
-            ws, wsb = workspaces.get(max(need, 256), dev, so)
-            check(fn(ctypes.cast(items, ctypes.c_void_p), hi - lo, ws, wsb, s), fn.__name__)
+    fn = _entry("sort_by_key", kt, vt, "copy_batch")
+    sizes = [k.numel() for k in in_keys]
+    rows = [(k.data_ptr(), v.data_ptr(), ok.data_ptr(), ov.data_ptr(), n)
+            for k, v, ok, ov, n in zip(in_keys, in_vals, out_keys, out_vals, sizes)]
+    for lo, hi in _chunks(len(rows)):
+        _issue(fn, dev, stream, "sort_by_key", kt, vt, sizes[lo:hi], "5Q", rows[lo:hi])
     return out_keys, out_vals

@@ -62,6 +62,7 @@ constexpr size_t merge_smem_bytes() {
 template <typename K>
 __global__ void merge_partition_kernel(const K *a, uint64_t na, const K *b, uint64_t nb, uint64_t tile,
                                        uint64_t num_parts, uint64_t *parts) {
+  grid_dependency_wait();
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= num_parts) return;
   const uint64_t total = na + nb;
@@ -198,6 +199,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     s_abort = 0;
   }
   __syncthreads();
+  grid_dependency_wait();
 
   // tiles of this CTA: first + i for i < mine (the grid is no larger than the tile count)
   const uint64_t first = args.tiles * blockIdx.x / G, mine = args.tiles * (blockIdx.x + 1) / G - first;
@@ -518,14 +520,14 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   if (tiles / kPerCta >= grid) {
     uint64_t *parts = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(d_ws) + kHeaderBytes);
     const uint64_t np = tiles + 1;
-    merge_partition_kernel<K><<<(unsigned)((np + 255) / 256), 256, 0, stream>>>(a, na, b, nb, C::TILE, np, parts);
-    if ((st = host::launch_status()) != BK_OK) return st;
+    st = host::launch_overlapped(merge_partition_kernel<K>, (unsigned)((np + 255) / 256), 256, 0, stream, 1, a, na, b, nb,
+                                 (uint64_t)C::TILE, np, parts);
+    if (st != BK_OK) return st;
     args.parts = parts;
   }
   const host::DebugFault dbg = host::debug_fault();
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
-  merge_kernel<K, P><<<grid, kMergeThreads, smem, stream>>>(args, hdr, limit);
-  return host::launch_status();
+  return host::launch_overlapped(merge_kernel<K, P>, grid, kMergeThreads, smem, stream, 1, args, hdr, limit);
 }
 
 size_t merge_workspace_bytes(int key_dtype, int value_dtype, uint64_t n) {

@@ -445,7 +445,7 @@ constexpr uint64_t kRsPlanMinN = 1ull << 22;
 // samples^2: the upper digits alone are sorted by up to an average of about 8.
 __device__ __forceinline__ RsPlan rs_plan(const RsPlanWs *plan, uint64_t n) {
   if (plan == nullptr) return kPlanFull;
-  const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(plan));
+  const uint4 w = ld_cg_v4(plan);
   if (w.z != 0u) return kPlanRescue;
   return (uint64_t)w.x * n <= 4ull * kRsSamples * kRsSamples ? kPlanUpper : kPlanFull;
 }
@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(kRsSampleThreads) rs_sample_kernel(const K *ke
     h = (h ^ (h >> 13)) * 0xc2b2ae35u;
     return h ^ (h >> 16);
   };
+  grid_dependency_wait();
   const unsigned int me = blockIdx.x * kRsSampleThreads + threadIdx.x;
   const uint64_t window = (uint64_t)mixed(blockIdx.x) * (n - kRsSampleWindow) >> 32;
   const uint32_t at_key = threadIdx.x * STRIDE + mixed(me + kRsSampleCtas) % STRIDE;
@@ -515,6 +516,7 @@ template <typename K, typename P>
 __global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *vals, uint32_t n, RsPlanWs *plan) {
   constexpr int WARPS = kRsFixThreads / 32, LEN = kRsFixChunk + kRsFixHalo, PER = LEN / 32;
   using V = typename std::conditional<has_payload<P>(), P, char>::type;
+  grid_dependency_wait();
   if (rs_plan(plan, n) == kPlanFull) return;
   // the keys' halves (up[-1]: of the key before the chunk); later, in the same
   // place, the keys that move, at their new places
@@ -683,6 +685,7 @@ __global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid
                                                                     unsigned int groups, unsigned int *hist,
                                                                     uint4 *status, const RsPlanWs *plan,
                                                                     bool rescue) {
+  grid_dependency_wait();
   const RsPlan p = rs_plan(plan, plan != nullptr ? src.group(0).n : 0);
   if (rescue) {
     if (p == kPlanRescue) rs_count_digits<K, P, Src, C, 0, 4>(src, groups, hist);
@@ -868,6 +871,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   __shared__ __align__(8) uint64_t s_group_bar;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned int me = rs_cluster_rank();
+  grid_dependency_wait();
   const int pass = rs_launch_digit(launch, plan, plan != nullptr ? src.group(0).n : 0);  // the digit
   if (pass < 0) return;
   const bool odd = launch & 1;
@@ -1104,6 +1108,7 @@ __global__ void __launch_bounds__(kRsClThreads, 1) rs_cluster_kernel(K *keys, P 
   __shared__ unsigned int s_dst[kRsBins];           // output position of staged position 0 for digit d
   __shared__ unsigned int s_scan[2 * (kRsBins / 32)];  // the two digit scans' warp totals
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_dependency_wait();
   const uint32_t me = rs_cluster_rank(), csize = rs_cluster_size();
   const uint32_t base = me * (uint32_t)TILE;
   const int count = (int)((n - base) < (uint32_t)TILE ? (n - base) : (uint32_t)TILE);
@@ -1125,8 +1130,8 @@ __global__ void __launch_bounds__(kRsClThreads, 1) rs_cluster_kernel(K *keys, P 
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
       const bool ok = elem(j) < count;
-      k[j] = ok ? __ldcg(in_k + base + elem(j)) : K();
-      if constexpr (has_payload<P>()) v[j] = ok ? __ldcg(in_v + base + elem(j)) : P();
+      k[j] = ok ? ld_cg(in_k + base + elem(j)) : K();
+      if constexpr (has_payload<P>()) v[j] = ok ? ld_cg(in_v + base + elem(j)) : P();
     }
     uint32_t dig4[ITEMS / 4];
 #pragma unroll
@@ -1240,19 +1245,8 @@ template <typename K, typename P, int ITEMS>
 int rs_cluster_launch(K *keys, P *vals, K *tk, P *tv, uint64_t n, cudaStream_t stream) {
   constexpr uint64_t TILE = (uint64_t)kRsClThreads * ITEMS;
   const unsigned c = (unsigned)((n + TILE - 1) / TILE);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(c);
-  cfg.blockDim = dim3(kRsClThreads);
-  cfg.dynamicSmemBytes = rs_cluster_smem_bytes<K, P, ITEMS>();
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = c;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return host::from_cuda(cudaLaunchKernelEx(&cfg, rs_cluster_kernel<K, P, ITEMS>, keys, vals, tk, tv, (uint32_t)n));
+  return host::launch_overlapped(rs_cluster_kernel<K, P, ITEMS>, c, kRsClThreads, rs_cluster_smem_bytes<K, P, ITEMS>(),
+                                 stream, c, keys, vals, tk, tv, (uint32_t)n);
 }
 
 // CTAs a group: four (eight leave up to an eighth of the SMs' room for CTAs
@@ -1321,25 +1315,6 @@ size_t radix_sort_batch_ws_bytes(const uint64_t *sizes, uint32_t count) {
   return RsLayout<K, P>(sz, m).total;
 }
 
-// Launch configuration of a pass: `clusters` clusters of C CTAs.
-template <typename K, typename P, int C>
-struct RsPassConfig {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  RsPassConfig(unsigned clusters, cudaStream_t stream) {
-    cfg.gridDim = dim3(clusters * C);
-    cfg.blockDim = dim3(RsCfg<K, P>::CTA_THREADS);
-    cfg.dynamicSmemBytes = rs_smem_bytes<K, P>();
-    cfg.stream = stream;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-  }
-};
-
 // The passes over `src` (one array or a batch).
 template <typename K, typename P, typename Src, int C>
 int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream_t stream) {
@@ -1356,8 +1331,18 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
   st = host::once_per_device<PassSite>(&clusters, [&](int *out) -> int {
     int e = host::set_smem_attrs(pass_kern, rs_smem_bytes<K, P>());
     if (e != BK_OK) return e;
-    RsPassConfig<K, P, C> pc(1, nullptr);
-    if ((e = host::from_cuda(cudaOccupancyMaxActiveClusters(out, pass_kern, &pc.cfg))) != BK_OK) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(RsCfg<K, P>::CTA_THREADS);
+    cfg.dynamicSmemBytes = rs_smem_bytes<K, P>();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if ((e = host::from_cuda(cudaOccupancyMaxActiveClusters(out, pass_kern, &cfg))) != BK_OK) return e;
     return *out > 0 ? BK_OK : BK_ERR_UNSUPPORTED;
   });
   if (st != BK_OK) return st;
@@ -1377,35 +1362,35 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
       host::KernelSetup fs;
       if ((st = host::kernel_setup<FixSite>(rs_fix_kernel<K, P>, kRsFixThreads, 0, &fs)) != BK_OK) return st;
       fix_ctas = (int)fs.resident_ctas;
-      rs_sample_kernel<K><<<kRsSampleCtas, kRsSampleThreads, 0, stream>>>(
-          src.keys, (uint32_t)src.n, reinterpret_cast<unsigned int *>(ws + L.samples), plan);
-      if ((st = host::launch_status()) != BK_OK) return st;
+      st = host::launch_overlapped(rs_sample_kernel<K>, kRsSampleCtas, kRsSampleThreads, 0, stream, 1,
+                                   (const K *)src.keys, (uint32_t)src.n,
+                                   reinterpret_cast<unsigned int *>(ws + L.samples), plan);
+      if (st != BK_OK) return st;
     }
   }
   const uint64_t tiles = L.groups * C;
   const unsigned hist_ctas = (unsigned)(tiles < hs.resident_ctas ? tiles : hs.resident_ctas);
-  hist_kern<<<hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream>>>(
-      src, groups, hist, reinterpret_cast<uint4 *>(ws + L.status[0]), plan, false);
-  if ((st = host::launch_status()) != BK_OK) return st;
+  auto count = [&](bool rescue) {
+    return host::launch_overlapped(hist_kern, hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream, 1, src, groups, hist,
+                                   reinterpret_cast<uint4 *>(ws + L.status[0]), (const RsPlanWs *)plan, rescue);
+  };
+  if ((st = count(false)) != BK_OK) return st;
   const unsigned used = groups < (unsigned)clusters ? groups : (unsigned)clusters;
-  RsPassConfig<K, P, C> pc(used, stream);
   // L2 prefetch distance: the table's number of residencies ahead (0: none)
   const tune::Knobs kn = tune::knobs_for(tune::kSort, RsCfg<K, P>::BYTES, L.groups * C * RsCfg<K, P>::TILE);
   const unsigned ahead = used * (unsigned)kn.prefetch;
   const int launches = plan != nullptr ? 12 : rs_passes<K>();
   for (int p = 0; p < launches; ++p) {
-    st = host::from_cuda(cudaLaunchKernelEx(&pc.cfg, pass_kern, src, p, (const RsPlanWs *)plan, groups,
-                                            (const unsigned int *)hist, tickets,
-                                            reinterpret_cast<unsigned int *>(ws + L.status[p & 1]),
-                                            reinterpret_cast<unsigned int *>(ws + L.status[(p & 1) ^ 1]), hdr, ahead, limit));
+    st = host::launch_overlapped(pass_kern, used * C, RsCfg<K, P>::CTA_THREADS, rs_smem_bytes<K, P>(), stream, C, src, p,
+                                 (const RsPlanWs *)plan, groups, (const unsigned int *)hist, tickets,
+                                 reinterpret_cast<unsigned int *>(ws + L.status[p & 1]),
+                                 reinterpret_cast<unsigned int *>(ws + L.status[(p & 1) ^ 1]), hdr, ahead, limit);
     if (st != BK_OK) return st;
     if constexpr (kPlanned) {
       if (plan != nullptr && p == 3) {
-        rs_fix_kernel<K, P><<<fix_ctas, kRsFixThreads, 0, stream>>>(src.keys, src.vals, (uint32_t)src.n, plan);
-        if ((st = host::launch_status()) != BK_OK) return st;
-        hist_kern<<<hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream>>>(
-            src, groups, hist, reinterpret_cast<uint4 *>(ws + L.status[0]), plan, true);
-        if ((st = host::launch_status()) != BK_OK) return st;
+        st = host::launch_overlapped(rs_fix_kernel<K, P>, (unsigned)fix_ctas, kRsFixThreads, 0, stream, 1, src.keys,
+                                     src.vals, (uint32_t)src.n, plan);
+        if (st != BK_OK || (st = count(true)) != BK_OK) return st;
       }
     }
   }

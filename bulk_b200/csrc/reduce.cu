@@ -36,9 +36,9 @@ size_t reduce_ws_bytes(int sm_count) {
 }
 
 template <typename T, typename Op>
-__global__ void __launch_bounds__(kReduceThreads, 4) reduce_kernel(const T *__restrict__ in, uint64_t head, uint64_t nvec,
-                                                                 uint64_t tail, T init, T *__restrict__ out,
-                                                                 T *__restrict__ partials, WsHeader *hdr) {
+__global__ void __launch_bounds__(kReduceThreads, 4) reduce_kernel(const T *in, uint64_t head, uint64_t nvec,
+                                                                 uint64_t tail, T init, T *out,
+                                                                 T *partials, WsHeader *hdr) {
   constexpr int V = ReduceLayout<T>::V;
   constexpr int U = kReduceUnroll;
   constexpr int A = 4;  // accumulator vectors: load u folds into acc[u % A]
@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(kReduceThreads, 4) reduce_kernel(const T *__re
     for (int j = 0; j < V; ++j) acc[a][j] = Op::identity();
 
   const int tid = threadIdx.x;
+  grid_dependency_wait();
   const uint4 *vin = reinterpret_cast<const uint4 *>(in + head);
   const uint64_t stride = (uint64_t)gridDim.x * kReduceThreads;
   uint64_t v = (uint64_t)blockIdx.x * kReduceThreads + tid;
@@ -157,8 +158,8 @@ int reduce_launch(const T *d_in, uint64_t n, T init, T *d_out, void *d_ws, size_
 
   WsHeader *hdr = reinterpret_cast<WsHeader *>(d_ws);
   T *partials = reinterpret_cast<T *>(reinterpret_cast<char *>(d_ws) + reduce_partials_offset());
-  reduce_kernel<T, Op><<<(unsigned)grid, kReduceThreads, 0, stream>>>(d_in, head, nvec, tail, init, d_out, partials, hdr);
-  return host::launch_status();
+  return host::launch_overlapped(reduce_kernel<T, Op>, (unsigned)grid, kReduceThreads, 0, stream, 1, d_in, head, nvec, tail,
+                                 init, d_out, partials, hdr);
 }
 
 size_t reduce_workspace_bytes(int dtype, uint64_t /*n*/) {

@@ -116,6 +116,7 @@ size_t rbk_ws_bytes(uint64_t n) {
 
 template <typename Status>
 __global__ void rbk_init_kernel(Status st, size_t tiles, WsHeader *hdr) {
+  grid_dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t padded = align_up(tiles, (size_t)kLbPerLane);
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(kRbkThreads, RbkCfg<K, V>::CTAS) rbk_kernel(co
   __shared__ unsigned int s_q_in;
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_dependency_wait();
   auto abort_now = [&]() { *reinterpret_cast<volatile int *>(&s_abort) = 1; };
   auto aborted = [&]() -> bool { return *reinterpret_cast<volatile int *>(&s_abort) != 0; };
   auto buf = [&](int b) { return smem_raw + (size_t)b * C::BUF_BYTES; };
@@ -830,8 +832,8 @@ int rbk_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStrea
   WsHeader *hdr = reinterpret_cast<WsHeader *>(d_ws);
   auto status = C::Status::at(reinterpret_cast<char *>(d_ws) + kHeaderBytes, tiles);
   const unsigned init_grid = (unsigned)std::min<size_t>((tiles + 255) / 256 + 1, (size_t)di.sm_count * 8);
-  rbk_init_kernel<<<init_grid, 256, 0, stream>>>(status, tiles, hdr);
-  if ((st = host::launch_status()) != BK_OK) return st;
+  st = host::launch_overlapped(rbk_init_kernel<typename C::Status>, init_grid, 256, 0, stream, 1, status, tiles, hdr);
+  if (st != BK_OK) return st;
   const host::DebugFault dbg = host::debug_fault();
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
   const size_t smem = (size_t)C::NB * C::BUF_BYTES + 1024;  // + room to align the buffers to 1024 bytes
@@ -842,9 +844,8 @@ int rbk_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStrea
   const size_t per_sm = (size_t)std::min(std::max(kn.ctas_per_sm, 1), C::CTAS);
   const unsigned grid = (unsigned)std::min<size_t>(tiles, std::min<size_t>((size_t)di.sm_count * per_sm, kRbkMaxGrid));
   unsigned char *ring = reinterpret_cast<unsigned char *>(d_ws) + rbk_ring_offset<K, V>(tiles);
-  rbk_kernel<K, V, Src><<<grid, kRbkThreads, smem, stream>>>(src, status, hdr, ring, limit, dbg.skip_publish_tile,
-                                                            (unsigned)tiles);
-  return host::launch_status();
+  return host::launch_overlapped(rbk_kernel<K, V, Src>, grid, kRbkThreads, smem, stream, 1, src, status, hdr, ring, limit,
+                                 dbg.skip_publish_tile, (unsigned)tiles);
 }
 
 template <typename K, typename V>

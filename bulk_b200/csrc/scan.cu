@@ -57,6 +57,7 @@ __host__ __device__ inline Status scan_status_at(void *ws, size_t tiles) {
 // Clears the status words of `tiles` tiles and resets the tile ticket.
 template <typename Status>
 __global__ void lookback_init_kernel(Status st, size_t tiles, WsHeader *hdr) {
+  grid_dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t padded = align_up(tiles, (size_t)kLbPerLane);  // whole look-back groups
@@ -103,7 +104,7 @@ struct ScanOne {
     const bool t_tma = kSwz ? (base + cnt <= covered) : (tma != 0);
     // only the first tile uses init; a device-resident one was written before
     // this launch (stream order) and is read-only during it
-    const T iv = (t == 0u && init_ptr != nullptr) ? __ldg(init_ptr) : init;
+    const T iv = (t == 0u && init_ptr != nullptr) ? ld_cg(init_ptr) : init;
     return ScanTile<T>{in + base, out + base, cnt, t == 0u, t_tma, iv, t};
   }
   __device__ __forceinline__ const CUtensorMap *in_map() const { return &imap; }
@@ -254,6 +255,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
   __shared__ unsigned int s_q_in;        // entries queued
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_dependency_wait();
   auto abort_now = [&]() { *reinterpret_cast<volatile int *>(&s_abort) = 1; };
   auto aborted = [&]() -> bool { return *reinterpret_cast<volatile int *>(&s_abort) != 0; };
   auto buf = [&](int b) { return buf0 + b * TILE; };
@@ -640,8 +642,7 @@ int scan_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStre
   WsHeader *hdr = reinterpret_cast<WsHeader *>(d_ws);
   auto status = scan_status_at<typename C::Status>(d_ws, tiles);
   const unsigned init_grid = (unsigned)std::min<size_t>((tiles + 255) / 256, (size_t)di.sm_count * 8);
-  lookback_init_kernel<<<init_grid, 256, 0, stream>>>(status, tiles, hdr);
-  st = host::launch_status();
+  st = host::launch_overlapped(lookback_init_kernel<typename C::Status>, init_grid, 256, 0, stream, 1, status, tiles, hdr);
   if (st != BK_OK) return st;
   const host::DebugFault dbg = host::debug_fault();
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
@@ -652,9 +653,8 @@ int scan_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStre
   const tune::Knobs kn = tune::knobs_for(tune::kScan, (int)sizeof(T), (uint64_t)tiles * C::TILE);
   const unsigned grid =
       (unsigned)std::min<size_t>(tiles, (size_t)di.sm_count * (size_t)std::min(std::max(kn.ctas_per_sm, 1), 2));
-  scan_kernel<T, Op, Src><<<grid, kScanThreads, smem, stream>>>(src, status, hdr, limit, dbg.skip_publish_tile,
-                                                                (unsigned)tiles);
-  return host::launch_status();
+  return host::launch_overlapped(scan_kernel<T, Op, Src>, grid, kScanThreads, smem, stream, 1, src, status, hdr, limit,
+                                 dbg.skip_publish_tile, (unsigned)tiles);
 }
 
 // init_ptr: when not null, init is read from device memory at run time (so a

@@ -461,6 +461,14 @@ __device__ __forceinline__ int rs_launch_digit(int launch, const RsPlanWs *plan,
   return block == 1 ? i : 4 + i;
 }
 
+// Clears the counts, tickets and sample (a kernel, not a memset, so that its
+// launch and its successor's overlap as all others here do).
+__global__ void rs_zero_kernel(uint4 *p, uint32_t vecs) {
+  grid_dependency_wait();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += gridDim.x * blockDim.x)
+    p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Every CTA takes one key from each 128th of a random window of 65,536 keys
 // and enters its upper half in a table of values seen (zeroed before; a zero
 // half is counted apart).  Windows, because reading 16,384 keys all over 2^26
@@ -609,7 +617,7 @@ __global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *v
 constexpr int kRsHistThreads = 1024;
 constexpr size_t kRsHistSmemBytes = 128 * 1024;
 
-// Counts digits [FIRST, FIRST + DIGITS).
+// Counts digits [FIRST, FIRST + DIGITS); the counters in shared memory start zeroed.
 template <typename K, typename P, typename Src, int C, int FIRST, int DIGITS>
 __device__ __forceinline__ void rs_count_digits(const Src &src, unsigned int groups, unsigned int *hist) {
   constexpr int BINS = DIGITS * kRsBins, COPIES = (int)(kRsHistSmemBytes / 4) / BINS;
@@ -617,8 +625,6 @@ __device__ __forceinline__ void rs_count_digits(const Src &src, unsigned int gro
   constexpr int VEC = 16 / (int)sizeof(K), UNROLL = 4;
   extern __shared__ __align__(16) unsigned int rs_hist_smem[];
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < BINS * COPIES / 4; i += kRsHistThreads)
-    reinterpret_cast<uint4 *>(rs_hist_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
   unsigned int *col = rs_hist_smem + (lane & (COPIES - 1));
   auto add = [&](K key) {
     const auto u = RadixKey<K>::to(key);
@@ -685,6 +691,9 @@ __global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid
                                                                     unsigned int groups, unsigned int *hist,
                                                                     uint4 *status, const RsPlanWs *plan,
                                                                     bool rescue) {
+  extern __shared__ __align__(16) unsigned int rs_hist_smem[];
+  for (int i = threadIdx.x; i < (int)(kRsHistSmemBytes / 16); i += kRsHistThreads)
+    reinterpret_cast<uint4 *>(rs_hist_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
   grid_dependency_wait();
   const RsPlan p = rs_plan(plan, plan != nullptr ? src.group(0).n : 0);
   if (rescue) {
@@ -871,11 +880,29 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   __shared__ __align__(8) uint64_t s_group_bar;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned int me = rs_cluster_rank();
+  const bool odd = launch & 1;
+  const RsRanker ranker(s_table[warp], s_bits[warp]);
+
+  // ---- shared memory made ready while the kernel before this one ends
+  auto clear_counters = [&](int b) {
+    uint4 *z = reinterpret_cast<uint4 *>(&s_whist[b][0][0]);
+#pragma unroll
+    for (int i = tid; i < WARPS * kRsBins / 8; i += THREADS) z[i] = make_uint4(0u, 0u, 0u, 0u);
+  };
+  if (tid < THREADS) clear_counters(0);
+  if (tid == 0) {
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&s_cnt_bar[b], 1);
+      mbar_init(&s_base_bar[b], 1);
+    }
+    mbar_init(&s_group_bar, 1);
+    rs_fence_mbar_init();
+    mbar_arrive_expect_tx(&s_group_bar, 4);
+  }
+  rs_cluster_sync();  // every CTA of the cluster runs, its barriers ready, before anything is sent to it
   grid_dependency_wait();
   const int pass = rs_launch_digit(launch, plan, plan != nullptr ? src.group(0).n : 0);  // the digit
   if (pass < 0) return;
-  const bool odd = launch & 1;
-  const RsRanker ranker(s_table[warp], s_bits[warp]);
 
   auto elem = [&](int j) { return warp * 32 * ITEMS + j * 32 + lane; };
   K k[ITEMS];
@@ -896,22 +923,6 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   // whoever starts first.
   const unsigned int clusters = gridDim.x / C;
   const bool more = groups > clusters;
-  auto clear_counters = [&](int b) {
-    uint4 *z = reinterpret_cast<uint4 *>(&s_whist[b][0][0]);
-#pragma unroll
-    for (int i = tid; i < WARPS * kRsBins / 8; i += THREADS) z[i] = make_uint4(0u, 0u, 0u, 0u);
-  };
-  if (tid < THREADS) clear_counters(0);
-  if (tid == 0) {
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_cnt_bar[b], 1);
-      mbar_init(&s_base_bar[b], 1);
-    }
-    mbar_init(&s_group_bar, 1);
-    rs_fence_mbar_init();
-    mbar_arrive_expect_tx(&s_group_bar, 4);
-  }
-  rs_cluster_sync();  // every CTA of the cluster runs, its barriers ready, before anything is sent to it
   if (me == 0 && warp == 0) {
     unsigned int t = 0;
     if (lane == 0) t = atomicAdd(&tickets[launch], 1u);
@@ -1352,7 +1363,11 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
   const unsigned groups = (unsigned)L.groups;
   const host::DebugFault df = host::debug_fault();
   const unsigned long long limit = df.spin_limit_ns ? df.spin_limit_ns : host::kDefaultSpinLimitNs;
-  if ((st = host::from_cuda(cudaMemsetAsync(hist, 0, L.zero_bytes, stream))) != BK_OK) return st;
+  const uint32_t zero_vecs = (uint32_t)(L.zero_bytes / 16);
+  const unsigned zero_ctas = (zero_vecs + 1023) / 1024;
+  if ((st = host::launch_overlapped(rs_zero_kernel, zero_ctas, 256, 0, stream, 1, reinterpret_cast<uint4 *>(hist),
+                                    zero_vecs)) != BK_OK)
+    return st;
   RsPlanWs *plan = nullptr;
   int fix_ctas = 0;
   if constexpr (kPlanned) {

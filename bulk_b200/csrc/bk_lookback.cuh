@@ -71,6 +71,33 @@ struct TileStatus {
   }
 };
 
+// Clears the status words of `tiles` tiles (whole look-back groups) and the
+// ticket, by every thread of a grid.
+template <typename Status>
+__device__ __forceinline__ void clear_status(const Status &st, size_t tiles, WsHeader *hdr) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t padded = align_up(tiles, (size_t)kLbPerLane);
+  for (size_t t = i; t < padded; t += (size_t)gridDim.x * blockDim.x) st.clear(t);
+  if (i == 0) hdr->tile_ticket = 0u;
+}
+template <typename Status>
+__global__ void lookback_init_kernel(Status st, size_t tiles, WsHeader *hdr) {
+  grid_dependency_wait();
+  clear_status(st, tiles, hdr);
+}
+
+// Arrays of up to this many tiles run as one thread-block cluster (portable
+// size), a CTA a tile.  The CTAs clear the status words themselves and meet
+// before the first of them takes a ticket, so no kernel has to clear them
+// first: one launch less a call (a scan of 50,021 i32, output allocated, on a
+// B200 box: 8.0 us a call against 10.0; the same 6 us of device time).
+constexpr unsigned kOneClusterTiles = 8;
+template <typename Status>
+__device__ __forceinline__ void clear_status_in_cluster(const Status &st, size_t tiles, WsHeader *hdr) {
+  clear_status(st, tiles, hdr);
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Ordered warp reduction: lane 0 receives v[31] (+) ... (+) v[1] (+) v[0]
 // (higher lanes hold earlier tiles), valid for non-commutative operators.
 template <typename P, typename Op>

@@ -114,16 +114,6 @@ size_t rbk_ws_bytes(uint64_t n) {
   return rbk_ws_for_tiles<K, V>(rbk_num_tiles<K, V>(n));
 }
 
-template <typename Status>
-__global__ void rbk_init_kernel(Status st, size_t tiles, WsHeader *hdr) {
-  grid_dependency_wait();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const size_t padded = align_up(tiles, (size_t)kLbPerLane);
-  for (size_t t = i; t < padded; t += stride) st.clear(t);
-  if (i == 0) hdr->tile_ticket = 0u;
-}
-
 template <typename V>
 __global__ void write_count_kernel(uint64_t *d_num_out) { *d_num_out = 0; }
 
@@ -459,7 +449,8 @@ template <typename K, typename V, typename Src>
 __global__ void __launch_bounds__(kRbkThreads, RbkCfg<K, V>::CTAS) rbk_kernel(const __grid_constant__ Src src,
                                                              typename RbkCfg<K, V>::Status st, WsHeader *hdr,
                                                              unsigned char *ring, unsigned long long spin_limit_ns,
-                                                             long long skip_publish_tile, unsigned int num_tiles) {
+                                                             long long skip_publish_tile, unsigned int num_tiles,
+                                                             bool one_cluster) {
   using C = RbkCfg<K, V>;
   using P = typename C::P;
   constexpr bool SWZ = Src::kSwz;
@@ -487,6 +478,7 @@ __global__ void __launch_bounds__(kRbkThreads, RbkCfg<K, V>::CTAS) rbk_kernel(co
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   grid_dependency_wait();
+  if (one_cluster) clear_status_in_cluster(st, num_tiles, hdr);
   auto abort_now = [&]() { *reinterpret_cast<volatile int *>(&s_abort) = 1; };
   auto aborted = [&]() -> bool { return *reinterpret_cast<volatile int *>(&s_abort) != 0; };
   auto buf = [&](int b) { return smem_raw + (size_t)b * C::BUF_BYTES; };
@@ -831,9 +823,12 @@ int rbk_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStrea
   if (st != BK_OK) return st;
   WsHeader *hdr = reinterpret_cast<WsHeader *>(d_ws);
   auto status = C::Status::at(reinterpret_cast<char *>(d_ws) + kHeaderBytes, tiles);
-  const unsigned init_grid = (unsigned)std::min<size_t>((tiles + 255) / 256 + 1, (size_t)di.sm_count * 8);
-  st = host::launch_overlapped(rbk_init_kernel<typename C::Status>, init_grid, 256, 0, stream, 1, status, tiles, hdr);
-  if (st != BK_OK) return st;
+  const bool one_cluster = tiles <= kOneClusterTiles;
+  if (!one_cluster) {
+    const unsigned init_grid = (unsigned)std::min<size_t>((tiles + 255) / 256 + 1, (size_t)di.sm_count * 8);
+    st = host::launch_overlapped(lookback_init_kernel<typename C::Status>, init_grid, 256, 0, stream, 1, status, tiles, hdr);
+    if (st != BK_OK) return st;
+  }
   const host::DebugFault dbg = host::debug_fault();
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
   const size_t smem = (size_t)C::NB * C::BUF_BYTES + 1024;  // + room to align the buffers to 1024 bytes
@@ -844,8 +839,8 @@ int rbk_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStrea
   const size_t per_sm = (size_t)std::min(std::max(kn.ctas_per_sm, 1), C::CTAS);
   const unsigned grid = (unsigned)std::min<size_t>(tiles, std::min<size_t>((size_t)di.sm_count * per_sm, kRbkMaxGrid));
   unsigned char *ring = reinterpret_cast<unsigned char *>(d_ws) + rbk_ring_offset<K, V>(tiles);
-  return host::launch_overlapped(rbk_kernel<K, V, Src>, grid, kRbkThreads, smem, stream, 1, src, status, hdr, ring, limit,
-                                 dbg.skip_publish_tile, (unsigned)tiles);
+  return host::launch_overlapped(rbk_kernel<K, V, Src>, grid, kRbkThreads, smem, stream, one_cluster ? grid : 1u, src,
+                                 status, hdr, ring, limit, dbg.skip_publish_tile, (unsigned)tiles, one_cluster);
 }
 
 template <typename K, typename V>

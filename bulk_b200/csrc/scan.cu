@@ -54,17 +54,6 @@ __host__ __device__ inline Status scan_status_at(void *ws, size_t tiles) {
   return Status::at(reinterpret_cast<char *>(ws) + kHeaderBytes, tiles);
 }
 
-// Clears the status words of `tiles` tiles and resets the tile ticket.
-template <typename Status>
-__global__ void lookback_init_kernel(Status st, size_t tiles, WsHeader *hdr) {
-  grid_dependency_wait();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const size_t padded = align_up(tiles, (size_t)kLbPerLane);  // whole look-back groups
-  for (size_t t = i; t < padded; t += stride) st.clear(t);
-  if (i == 0) hdr->tile_ticket = 0u;
-}
-
 // Where one tile lives.
 template <typename T>
 struct ScanTile {
@@ -233,7 +222,8 @@ template <typename T, typename Op, typename Src>
 __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_constant__ Src src,
                                                                typename ScanCfg<T>::Status st, WsHeader *hdr,
                                                                unsigned long long spin_limit_ns,
-                                                               long long skip_publish_tile, unsigned int num_tiles) {
+                                                               long long skip_publish_tile, unsigned int num_tiles,
+                                                               bool one_cluster) {
   using C = ScanCfg<T>;
   constexpr int V = C::V, TILE = C::TILE, R = kScanRowsPerWarp, NB = kScanBufs, Q = kScanQueue;
   constexpr unsigned int NONE = 0xffffffffu;
@@ -256,6 +246,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) scan_kernel(const __grid_cons
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   grid_dependency_wait();
+  if (one_cluster) clear_status_in_cluster(st, num_tiles, hdr);
   auto abort_now = [&]() { *reinterpret_cast<volatile int *>(&s_abort) = 1; };
   auto aborted = [&]() -> bool { return *reinterpret_cast<volatile int *>(&s_abort) != 0; };
   auto buf = [&](int b) { return buf0 + b * TILE; };
@@ -641,9 +632,12 @@ int scan_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStre
   if (st != BK_OK) return st;
   WsHeader *hdr = reinterpret_cast<WsHeader *>(d_ws);
   auto status = scan_status_at<typename C::Status>(d_ws, tiles);
-  const unsigned init_grid = (unsigned)std::min<size_t>((tiles + 255) / 256, (size_t)di.sm_count * 8);
-  st = host::launch_overlapped(lookback_init_kernel<typename C::Status>, init_grid, 256, 0, stream, 1, status, tiles, hdr);
-  if (st != BK_OK) return st;
+  const bool one_cluster = tiles <= kOneClusterTiles;
+  if (!one_cluster) {
+    const unsigned init_grid = (unsigned)std::min<size_t>((tiles + 255) / 256, (size_t)di.sm_count * 8);
+    st = host::launch_overlapped(lookback_init_kernel<typename C::Status>, init_grid, 256, 0, stream, 1, status, tiles, hdr);
+    if (st != BK_OK) return st;
+  }
   const host::DebugFault dbg = host::debug_fault();
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
   const size_t smem = (size_t)kScanBufs * C::TILE_BYTES + 1024;  // + room to align the buffers to 1024 bytes
@@ -653,8 +647,8 @@ int scan_run(const Src &src, size_t tiles, void *d_ws, size_t ws_bytes, cudaStre
   const tune::Knobs kn = tune::knobs_for(tune::kScan, (int)sizeof(T), (uint64_t)tiles * C::TILE);
   const unsigned grid =
       (unsigned)std::min<size_t>(tiles, (size_t)di.sm_count * (size_t)std::min(std::max(kn.ctas_per_sm, 1), 2));
-  return host::launch_overlapped(scan_kernel<T, Op, Src>, grid, kScanThreads, smem, stream, 1, src, status, hdr, limit,
-                                 dbg.skip_publish_tile, (unsigned)tiles);
+  return host::launch_overlapped(scan_kernel<T, Op, Src>, grid, kScanThreads, smem, stream, one_cluster ? grid : 1u, src,
+                                 status, hdr, limit, dbg.skip_publish_tile, (unsigned)tiles, one_cluster);
 }
 
 // init_ptr: when not null, init is read from device memory at run time (so a

@@ -21,7 +21,8 @@
 //
 // A single array of up to 131,072 keys is sorted instead by one launch of one
 // thread-block cluster whose CTAs exchange their digit counts through
-// distributed shared memory (rs_cluster_kernel below).
+// distributed shared memory (rs_cluster_kernel below), of up to 4096 keys by
+// one CTA (rs_block_kernel).
 #include <type_traits>
 
 #include "bk_common.cuh"
@@ -1077,24 +1078,26 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
 }
 
 // ---------------------------------------------------------------------------
-// Small arrays (up to 16 tiles of 4096 or 8192 keys): every pass in one launch
-// of one thread-block cluster, one CTA per tile.  The CTAs exchange their digit counts through
+// Small arrays (up to 16 tiles): every pass in one launch of one thread-block
+// cluster, one CTA per tile.  A pass ranks a tile's keys at the rate of the
+// SM's shared-memory pipe (about 31 accesses of a warp for 32 keys), so the
+// tile is the smallest that 16 CTAs cover: 1024, 2048 or 4096 keys of 256, 512
+// or 1024 threads, then 8192.  The CTAs exchange their digit counts through
 // distributed shared memory (each reads every other CTA's 256 counts across
 // the cluster) instead of a count scan in global memory, and a cluster barrier
 // takes the place of each kernel boundary: two barriers a pass replace the
-// three launches a pass of the global-memory path takes.  The keys move
+// launches of the global-memory path.  The keys move
 // between passes through the workspace temporaries, which stay in L2 at these
 // sizes (storing each key straight into the owning CTA's shared memory was
 // measured slower: 42.9 against 32.8 us for 2^16 u32/u32 keys on a B200).
 constexpr int kRsClusterMax = 16;  // CTAs (non-portable above 8)
-constexpr int kRsClThreads = 1024;  // four or eight items a thread: short ranking chains, 32 warps an SM
 
 // Shared memory of a cluster-sort CTA of ITEMS items a thread: one tile
-// (1024 * ITEMS keys and payloads), or the ranking tables that lie in the same place.
-template <typename K, typename P, int ITEMS>
+// (TH * ITEMS keys and payloads), or the ranking tables that lie in the same place.
+template <typename K, typename P, int TH, int ITEMS>
 constexpr size_t rs_cluster_smem_bytes() {
-  constexpr size_t tile = align_up(sizeof(K) * kRsClThreads * ITEMS, 16) + (size_t)payload_bytes<P>() * kRsClThreads * ITEMS;
-  constexpr size_t tables = 256 + (size_t)(kRsClThreads / 32) * (512 + 128);
+  constexpr size_t tile = align_up(sizeof(K) * TH * ITEMS, 16) + (size_t)payload_bytes<P>() * TH * ITEMS;
+  constexpr size_t tables = 256 + (size_t)(TH / 32) * (512 + 128);
   return tile > tables ? tile : tables;
 }
 
@@ -1107,9 +1110,9 @@ constexpr size_t rs_cluster_smem_bytes() {
 // cluster barrier after the writes (release / acquire at cluster scope) makes
 // them visible to the CTA that reads that tile next.  Even passes end in the
 // array, so the last one leaves the result in place.
-template <typename K, typename P, int ITEMS>
-__global__ void __launch_bounds__(kRsClThreads, 1) rs_cluster_kernel(K *keys, P *vals, K *tk, P *tv, uint32_t n) {
-  constexpr int WARPS = kRsClThreads / 32, TILE = kRsClThreads * ITEMS;
+template <typename K, typename P, int TH, int ITEMS>
+__global__ void __launch_bounds__(TH, 1) rs_cluster_kernel(K *keys, P *vals, K *tk, P *tv, uint32_t n) {
+  constexpr int WARPS = TH / 32, TILE = TH * ITEMS;
   constexpr size_t VOFF = align_up(sizeof(K) * TILE, 16);
   extern __shared__ __align__(16) unsigned char rs_cl_smem[];
   K *sk = reinterpret_cast<K *>(rs_cl_smem);  // the tile in digit order
@@ -1123,7 +1126,7 @@ __global__ void __launch_bounds__(kRsClThreads, 1) rs_cluster_kernel(K *keys, P 
   const uint32_t me = rs_cluster_rank(), csize = rs_cluster_size();
   const uint32_t base = me * (uint32_t)TILE;
   const int count = (int)((n - base) < (uint32_t)TILE ? (n - base) : (uint32_t)TILE);
-  for (int i = tid; i < WARPS * kRsBins / 8; i += kRsClThreads)
+  for (int i = tid; i < WARPS * kRsBins / 8; i += TH)
     reinterpret_cast<uint4 *>(&s_whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
   // the ranking tables lie in the staging area, which is written after every warp has ranked its keys
@@ -1197,9 +1200,9 @@ __global__ void __launch_bounds__(kRsClThreads, 1) rs_cluster_kernel(K *keys, P 
       if constexpr (has_payload<P>()) sv[pos] = v[j];
     }
     __syncthreads();
-    for (int i = tid; i < WARPS * kRsBins / 8; i += kRsClThreads)
+    for (int i = tid; i < WARPS * kRsBins / 8; i += TH)
     reinterpret_cast<uint4 *>(&s_whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int p = tid; p < count; p += kRsClThreads) {
+    for (int p = tid; p < count; p += TH) {
       const K key = sk[p];
       const uint32_t g = s_dst[rs_digit(key, shift)] + (uint32_t)p;
       if (g < n) {
@@ -1212,13 +1215,13 @@ __global__ void __launch_bounds__(kRsClThreads, 1) rs_cluster_kernel(K *keys, P 
 }
 
 // Once per device: the largest cluster (16 or 8 CTAs, 0 for none) that the
-// cluster sort can be launched with, for tiles of 1024 * ITEMS keys.
-template <typename K, typename P, int ITEMS>
+// cluster sort can be launched with, for tiles of TH * ITEMS keys.
+template <typename K, typename P, int TH, int ITEMS>
 int rs_cluster_setup(int *max_ctas) {
   struct Site {};
   return host::once_per_device<Site>(max_ctas, [](int *mx) -> int {
-    auto kern = rs_cluster_kernel<K, P, ITEMS>;
-    constexpr size_t smem = rs_cluster_smem_bytes<K, P, ITEMS>();
+    auto kern = rs_cluster_kernel<K, P, TH, ITEMS>;
+    constexpr size_t smem = rs_cluster_smem_bytes<K, P, TH, ITEMS>();
     int st;
     if ((st = host::set_smem_attrs(kern, smem)) != BK_OK) return st;
     *mx = 0;
@@ -1227,7 +1230,7 @@ int rs_cluster_setup(int *max_ctas) {
     for (int c : {kRsClusterMax, 8}) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)c);
-      cfg.blockDim = dim3(kRsClThreads);
+      cfg.blockDim = dim3(TH);
       cfg.dynamicSmemBytes = smem;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1250,13 +1253,13 @@ int rs_cluster_setup(int *max_ctas) {
   });
 }
 
-// The cluster sort of n elements (n <= 1024 * ITEMS * max_ctas), one launch;
+// The cluster sort of n elements (n <= TH * ITEMS * max_ctas), one launch;
 // tk / tv are the workspace temporaries of n elements.
-template <typename K, typename P, int ITEMS>
+template <typename K, typename P, int TH, int ITEMS>
 int rs_cluster_launch(K *keys, P *vals, K *tk, P *tv, uint64_t n, cudaStream_t stream) {
-  constexpr uint64_t TILE = (uint64_t)kRsClThreads * ITEMS;
+  constexpr uint64_t TILE = (uint64_t)TH * ITEMS;
   const unsigned c = (unsigned)((n + TILE - 1) / TILE);
-  return host::launch_overlapped(rs_cluster_kernel<K, P, ITEMS>, c, kRsClThreads, rs_cluster_smem_bytes<K, P, ITEMS>(),
+  return host::launch_overlapped(rs_cluster_kernel<K, P, TH, ITEMS>, c, TH, rs_cluster_smem_bytes<K, P, TH, ITEMS>(),
                                  stream, c, keys, vals, tk, tv, (uint32_t)n);
 }
 
@@ -1412,6 +1415,8 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
   return BK_OK;
 }
 
+constexpr int kNoCluster = 1 << 30;  // no status
+
 template <typename K, typename P>
 int radix_sort_launch(K *keys, P *vals, uint64_t n, void *d_ws, size_t ws_bytes, cudaStream_t stream) {
   host::DeviceInfo di;
@@ -1429,13 +1434,19 @@ int radix_sort_launch(K *keys, P *vals, uint64_t n, void *d_ws, size_t ws_bytes,
   char *ws = reinterpret_cast<char *>(d_ws);
   K *tk = reinterpret_cast<K *>(ws + L.tmp);
   P *tv = reinterpret_cast<P *>(ws + L.tmp + align_up(n * sizeof(K), 256));
-  // one cluster launch: four items a thread up to 16 tiles of 4096 keys (more
-  // CTAs, a shorter pass), eight up to 16 tiles of 8192
-  int cl4 = 0, cl8 = 0;
-  if ((st = rs_cluster_setup<K, P, 4>(&cl4)) != BK_OK) return st;
-  if (n <= (uint64_t)kRsClThreads * 4 * (uint64_t)cl4) return rs_cluster_launch<K, P, 4>(keys, vals, tk, tv, n, stream);
-  if ((st = rs_cluster_setup<K, P, 8>(&cl8)) != BK_OK) return st;
-  if (n <= (uint64_t)kRsClThreads * 8 * (uint64_t)cl8) return rs_cluster_launch<K, P, 8>(keys, vals, tk, tv, n, stream);
+  auto cluster = [&](auto th, auto items) -> int {  // the sort's status, or kNoCluster when n needs more CTAs
+    constexpr int TH = decltype(th)::value, ITEMS = decltype(items)::value;
+    int ctas = 0;
+    const int e = rs_cluster_setup<K, P, TH, ITEMS>(&ctas);
+    if (e != BK_OK) return e;
+    if (n > (uint64_t)TH * ITEMS * (uint64_t)ctas) return kNoCluster;
+    return rs_cluster_launch<K, P, TH, ITEMS>(keys, vals, tk, tv, n, stream);
+  };
+  using std::integral_constant;
+  if ((st = cluster(integral_constant<int, 256>(), integral_constant<int, 4>())) != kNoCluster) return st;
+  if ((st = cluster(integral_constant<int, 512>(), integral_constant<int, 4>())) != kNoCluster) return st;
+  if ((st = cluster(integral_constant<int, 1024>(), integral_constant<int, 4>())) != kNoCluster) return st;
+  if ((st = cluster(integral_constant<int, 1024>(), integral_constant<int, 8>())) != kNoCluster) return st;
   return radix_sort_run<K, P, RsOne<K, P>, kRsCtas>(RsOne<K, P>{keys, vals, tk, tv, n}, L, ws, stream);
 }
 
@@ -1449,6 +1460,226 @@ struct RsItem {
   P *vals;
   uint64_t n;
 };
+
+// ---------------------------------------------------------------------------
+// Arrays of up to kRsBlockMax keys: one CTA each, every pass in shared memory.
+// The keys and payloads go round through the staging area (ranked as above,
+// stored in digit order, read back); three barriers a pass.  Bound by the
+// SM's shared-memory pipe, as the cluster sort is, but with nothing exchanged,
+// and a CTA sees all keys: passes whose digit is the same in every key are
+// left out, and 8-byte keys whose upper halves mostly differ are sorted by
+// their upper digits, then their short runs of equal upper halves are put in
+// order in place (by counting, as rs_fix_kernel does).  On a B200, with the
+// block sort by merging before: u32/u32 1024 keys 5.6 us (22.5), 4096 11.8 (24.4);
+// u64/u32 1024 6.2 (18.4), 4096 15.9 (20.0; 22 where few upper halves and all
+// digits occur, so that all eight passes are needed).
+// ---------------------------------------------------------------------------
+constexpr int kRsBlockMax = 4096, kRsBlockItems = 4;
+
+template <typename K, typename P, int N>
+struct RsBlockItems {
+  const K *in_k[N];
+  const P *in_v[N];
+  K *out_k[N];
+  P *out_v[N];
+  uint32_t n[N];
+};
+
+template <typename K, typename P, int TH>
+constexpr size_t rs_block_smem_bytes() {
+  constexpr size_t tile = (size_t)TH * kRsBlockItems;
+  return 256 + (size_t)(TH / 32) * (512 + 128) + align_up(sizeof(K) * tile, 16) + (size_t)payload_bytes<P>() * tile;
+}
+
+template <typename K, typename P, int TH, int N>
+__global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__ RsBlockItems<K, P, N> items) {
+  constexpr int ITEMS = kRsBlockItems, WARPS = TH / 32, TILE = TH * ITEMS;
+  extern __shared__ __align__(16) unsigned char rs_bl_smem[];
+  __shared__ __align__(16) uint16_t s_whist[WARPS][kRsBins];  // per-warp digit counters, then staging starts (both x4)
+  __shared__ unsigned int s_scan[kRsBins / 32];
+  __shared__ unsigned int s_vary[2];  // bits that differ between keys: lower and upper halves
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned char *tables = rs_bl_smem + (256u - (smem_addr(rs_bl_smem) & 255u));
+  unsigned char *bits = tables + WARPS * 512;
+  K *sk = reinterpret_cast<K *>(bits + WARPS * 128);
+  P *sv = reinterpret_cast<P *>(reinterpret_cast<unsigned char *>(sk) + align_up(sizeof(K) * TILE, 16));
+  const RsRanker ranker(tables + warp * 512, bits + warp * 128);
+  uint4 *const mine = reinterpret_cast<uint4 *>(&s_whist[warp][0]) + lane;  // a warp clears its own counters
+  *mine = make_uint4(0u, 0u, 0u, 0u);
+  if (tid < 2) s_vary[tid] = 0u;
+  __syncthreads();
+  grid_dependency_wait();
+  const K *in_k = items.in_k[blockIdx.x];
+  const P *in_v = items.in_v[blockIdx.x];
+  const int count = (int)items.n[blockIdx.x];
+  auto elem = [&](int j) { return warp * 32 * ITEMS + j * 32 + lane; };
+  K k[ITEMS];
+  P v[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    k[j] = elem(j) < count ? in_k[elem(j)] : K();
+    if constexpr (has_payload<P>()) v[j] = elem(j) < count ? in_v[elem(j)] : P();
+  }
+  // the digits that differ between keys
+  unsigned int todo;
+  {
+    const auto first = RadixKey<K>::to(in_k[0]);
+    typename RadixKey<K>::U x = 0;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+      if (elem(j) < count) x |= RadixKey<K>::to(k[j]) ^ first;
+#pragma unroll
+    for (int h = 0; h < (int)sizeof(K) / 4; ++h) {
+      const unsigned int o = __reduce_or_sync(0xffffffffu, rs_word(x, 4 * h));
+      if (lane == 0 && o != 0u) atomicOr(&s_vary[h], o);
+    }
+    __syncthreads();
+    auto digits = [](unsigned int w) {
+      return (w & 0xffu ? 1u : 0u) | (w & 0xff00u ? 2u : 0u) | (w & 0xff0000u ? 4u : 0u) | (w & 0xff000000u ? 8u : 0u);
+    };
+    todo = digits(s_vary[0]);
+    if constexpr (sizeof(K) == 8) todo |= digits(s_vary[1]) << 4;
+  }
+  const unsigned int all = todo;
+  bool upper = false;  // the upper digits alone, to begin with
+  if constexpr (sizeof(K) == 8) {
+    // not where half of the warps see an upper half twice among 32 keys
+    const bool twice = __popc(__match_any_sync(0xffffffffu, rs_word(RadixKey<K>::to(k[0]), 4))) > 1 && elem(0) < count;
+    const bool warp_twice = __any_sync(0xffffffffu, twice);
+    const int warps = __syncthreads_count(lane == 0 && warp_twice);
+    upper = (all >> 4) != 0u && (all & 15u) != 0u && 2 * warps < (count + 127) / 128;
+  }
+  if (upper) todo &= 0xf0u;
+  while (todo != 0u) {
+    const int pass = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    // past the array's end the digit is 255: those items stay last
+    uint32_t dig4[1] = {rs_digits4(k, pass)};
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+      if (elem(j) >= count) dig4[0] |= 0xffu << (8 * j);
+    uint32_t rank2[ITEMS / 2];
+    ranker.rank<ITEMS>(s_whist[warp], dig4, rank2);
+    __syncthreads();
+    if (tid < kRsBins) {
+      unsigned int cnt = 0, total;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) cnt += s_whist[w][tid];
+      unsigned int run = rs_scan_digits(cnt, s_scan, total);
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        const unsigned int c = s_whist[w][tid];
+        s_whist[w][tid] = (uint16_t)run;
+        run += c;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = (dig4[0] >> (8 * j)) & 0xffu;
+      const uint32_t pos = (s_whist[warp][d] + ((rank2[j >> 1] >> (16 * (j & 1))) & 0xffffu)) >> 2;
+      sk[pos] = k[j];
+      if constexpr (has_payload<P>()) sv[pos] = v[j];
+    }
+    __syncwarp();
+    *mine = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      k[j] = sk[elem(j)];
+      if constexpr (has_payload<P>()) v[j] = sv[elem(j)];
+    }
+    if constexpr (sizeof(K) == 8) {
+      if (upper && todo == 0u) {
+        upper = false;
+        constexpr int LONGEST = 64;
+        int to[ITEMS];
+        bool move = false, redo = false;
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+          const int i = elem(j);
+          to[j] = -1;
+          if (i >= count) continue;
+          const uint64_t u = RadixKey<K>::to(k[j]);
+          auto same = [&](int q) { return (unsigned int)((RadixKey<K>::to(sk[q]) ^ u) >> 32) == 0u; };
+          int first = i, last = i, rank = 0;
+          while (first > 0 && last - first < LONGEST && same(first - 1)) {
+            --first;
+            rank += RadixKey<K>::to(sk[first]) <= u;
+          }
+          while (last + 1 < count && last - first < LONGEST && same(last + 1)) {
+            ++last;
+            rank += RadixKey<K>::to(sk[last]) < u;
+          }
+          if (last - first >= LONGEST) {
+            redo |= i > 0 && same(i - 1) && RadixKey<K>::to(sk[i - 1]) > u;
+          } else if (first + rank != i) {
+            to[j] = first + rank;
+            move = true;
+          }
+        }
+        redo = __syncthreads_or(redo);
+        if (__syncthreads_or(move)) {
+#pragma unroll
+          for (int j = 0; j < ITEMS; ++j) {
+            if (to[j] >= 0) {
+              sk[to[j]] = k[j];
+              if constexpr (has_payload<P>()) sv[to[j]] = v[j];
+            }
+          }
+          __syncthreads();
+#pragma unroll
+          for (int j = 0; j < ITEMS; ++j) {
+            k[j] = sk[elem(j)];
+            if constexpr (has_payload<P>()) v[j] = sv[elem(j)];
+          }
+        }
+        if (redo) todo = all;  // a long run out of order: all digits (equal keys are still in input order)
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    if (elem(j) < count) {
+      items.out_k[blockIdx.x][elem(j)] = k[j];
+      if constexpr (has_payload<P>()) items.out_v[blockIdx.x][elem(j)] = v[j];
+    }
+  }
+}
+
+template <typename K, typename P, int TH, int N>
+int rs_block_run(const RsBlockItems<K, P, N> &items, uint32_t count, cudaStream_t stream) {
+  struct Site {};
+  host::KernelSetup ks;
+  constexpr size_t smem = rs_block_smem_bytes<K, P, TH>();
+  const int st = host::kernel_setup<Site>(rs_block_kernel<K, P, TH, N>, TH, smem, &ks);
+  if (st != BK_OK) return st;
+  return host::launch_overlapped(rs_block_kernel<K, P, TH, N>, count, TH, smem, stream, 1, items);
+}
+
+// `count` arrays of 1 to kRsBlockMax keys each, checked by the caller.
+template <typename K, typename P>
+int radix_sort_blocks(const RsItem<K, P> *items, uint32_t count, cudaStream_t stream) {
+  auto run = [&](auto cap) {
+    RsBlockItems<K, P, decltype(cap)::value> b;
+    uint64_t longest = 0;
+    uint32_t m = 0;
+    for (uint32_t i = 0; i < count; ++i) {
+      if (items[i].n == 0) continue;
+      b.in_k[m] = items[i].in_keys;
+      b.in_v[m] = items[i].in_vals;
+      b.out_k[m] = items[i].keys;
+      b.out_v[m] = items[i].vals;
+      b.n[m++] = (uint32_t)items[i].n;
+      longest = items[i].n > longest ? items[i].n : longest;
+    }
+    if (m == 0) return (int)BK_OK;
+    return longest <= 1024   ? rs_block_run<K, P, 256, decltype(cap)::value>(b, m, stream)
+           : longest <= 2048 ? rs_block_run<K, P, 512, decltype(cap)::value>(b, m, stream)
+                             : rs_block_run<K, P, 1024, decltype(cap)::value>(b, m, stream);
+  };
+  return count == 1 ? run(std::integral_constant<int, 1>()) : run(std::integral_constant<int, kRsBatchMax>());
+}
 
 template <typename K, typename P>
 int radix_sort_batch_launch(const RsItem<K, P> *items, uint32_t count, void *d_ws, size_t ws_bytes,
@@ -1517,6 +1748,7 @@ int radix_sort_batch_launch(const RsItem<K, P> *items, uint32_t count, void *d_w
 #define BK_RS_INST_P(K, P)                                                                                  \
   template int radix_sort_launch<K, P>(K *, P *, uint64_t, void *, size_t, cudaStream_t);                  \
   template size_t radix_sort_ws_bytes<K, P>(uint64_t);                                                      \
+  template int radix_sort_blocks<K, P>(const RsItem<K, P> *, uint32_t, cudaStream_t);                       \
   template int radix_sort_batch_launch<K, P>(const RsItem<K, P> *, uint32_t, void *, size_t, cudaStream_t); \
   template size_t radix_sort_batch_ws_bytes<K, P>(const uint64_t *, uint32_t);
 #define BK_RS_INST(K)        \

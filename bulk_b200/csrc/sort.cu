@@ -37,7 +37,10 @@ int radix_sort_batch_launch(const RsItem<K, P> *items, uint32_t count, void *d_w
                             cudaStream_t stream);
 template <typename K, typename P>
 size_t radix_sort_batch_ws_bytes(const uint64_t *sizes, uint32_t count);
+template <typename K, typename P>
+int radix_sort_blocks(const RsItem<K, P> *items, uint32_t count, cudaStream_t stream);
 constexpr uint64_t kRadixMaxN = 1ull << 30;
+constexpr uint64_t kRadixBlockMax = 4096;  // keys of an array that one CTA sorts in shared memory
 
 constexpr int kBsThreads = 512;  // block sort
 constexpr int kMpThreads = 256;  // merge passes
@@ -331,12 +334,12 @@ size_t merge_sort_ws_bytes_t(uint64_t n) {
          align_up((mp_tiles + 1) * sizeof(uint64_t), 256);
 }
 
-// Which sort an array gets: one block-sort launch when it fits one block
-// tile (4 or 8 radix passes cost more than its merge rounds there), the radix
-// sort up to 2^30 elements, the merge sort above.
+// Which sort an array gets: the radix sort in one CTA up to kRadixBlockMax
+// keys, the radix sort over more CTAs up to 2^30 elements, the merge sort
+// above.
 template <typename K>
 bool use_radix(uint64_t n) {
-  return n > (uint64_t)SortCfg<K>::BS_TILE && n < kRadixMaxN;
+  return n > kRadixBlockMax && n < kRadixMaxN;
 }
 
 template <typename K, typename P>
@@ -397,6 +400,10 @@ int sort_launch(K *keys, P *vals, uint64_t n, void *d_ws, size_t ws_bytes, cudaS
   const uint64_t mp_tiles = (n + C::MP_TILE - 1) / C::MP_TILE;
   st = host::check_ws(d_ws, ws_bytes, sort_ws_bytes_t<K, P>(n));
   if (st != BK_OK) return st;
+  if (n <= kRadixBlockMax) {
+    const RsItem<K, P> item{keys, vals, keys, vals, n};
+    return radix_sort_blocks<K, P>(&item, 1, stream);
+  }
   char *ws = reinterpret_cast<char *>(d_ws) + kHeaderBytes;
   K *tk = reinterpret_cast<K *>(ws);
   ws += align_up(n * sizeof(K), 256);
@@ -458,15 +465,16 @@ size_t merge_sort_batch_ws_bytes_t(const uint64_t *sizes, uint32_t count) {
   return b;
 }
 
-// A batch uses the radix sort when all its arrays are below 2^30 elements
-// and one needs more than a block tile; otherwise the merge sort (a single
-// block-sort launch when every array fits one tile).
+// A batch uses the radix sort over groups of CTAs when all its arrays are
+// below 2^30 elements and one needs more than a block-sort tile; otherwise
+// each array has a CTA (the radix sort in shared memory when none is above
+// kRadixBlockMax keys, else the block sort), or the merge sort sorts them.
 template <typename K, typename P>
 bool sort_batch_radix(const uint64_t *sizes, uint32_t count) {
   bool any_large = false;
   for (uint32_t i = 0; i < count; ++i) {
     if (sizes[i] >= kRadixMaxN) return false;
-    any_large = any_large || use_radix<K>(sizes[i]);
+    any_large = any_large || sizes[i] > (uint64_t)SortCfg<K>::BS_TILE;
   }
   return any_large;
 }
@@ -530,6 +538,10 @@ int sort_batch_copy_launch(const SortCopyItem<K, P> *items, uint32_t count, void
   }
   st = host::check_ws(d_ws, ws_bytes, merge_sort_batch_ws_bytes_t<K, P>(sizes, count));
   if (st != BK_OK) return st;
+  uint64_t longest = 0;
+  for (uint32_t i = 0; i < count; ++i) longest = sizes[i] > longest ? sizes[i] : longest;
+  if (longest <= kRadixBlockMax)
+    return radix_sort_blocks<K, P>(reinterpret_cast<const RsItem<K, P> *>(items), count, stream);
   char *ws = reinterpret_cast<char *>(d_ws) + kHeaderBytes;
   int max_passes = 0;
   size_t bs_total = 0;

@@ -344,7 +344,11 @@ bool use_radix(uint64_t n) {
 
 template <typename K, typename P>
 size_t sort_ws_bytes_t(uint64_t n) {
-  return use_radix<K>(n) ? radix_sort_ws_bytes<K, P>(n) : merge_sort_ws_bytes_t<K, P>(n);
+  if (!use_radix<K>(n)) return merge_sort_ws_bytes_t<K, P>(n);
+  const size_t radix = radix_sort_ws_bytes<K, P>(n);
+  if (n > (uint64_t)SortCfg<K>::BS_TILE) return radix;
+  const size_t merge = merge_sort_ws_bytes_t<K, P>(n);  // a batch of this array alone sorts it as one block-sort tile
+  return radix > merge ? radix : merge;
 }
 
 template <typename Kern>
@@ -481,6 +485,7 @@ bool sort_batch_radix(const uint64_t *sizes, uint32_t count) {
 
 template <typename K, typename P>
 size_t sort_batch_ws_bytes_t(const uint64_t *sizes, uint32_t count) {
+  if (count == 1) return sort_ws_bytes_t<K, P>(sizes[0]);
   return sort_batch_radix<K, P>(sizes, count) ? radix_sort_batch_ws_bytes<K, P>(sizes, count)
                                               : merge_sort_batch_ws_bytes_t<K, P>(sizes, count);
 }

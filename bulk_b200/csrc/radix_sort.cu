@@ -373,7 +373,9 @@ struct RsOne {
   K *tk;
   P *tv;
   uint64_t n;
-  __device__ __forceinline__ RsGroup<K, P> group(unsigned int g) const {
+  static constexpr bool kMany = false;
+  __device__ __forceinline__ unsigned int find(unsigned int) const { return 0u; }
+  __device__ __forceinline__ RsGroup<K, P> group(unsigned int g, unsigned int = 0u) const {
     return RsGroup<K, P>{keys, vals, tk, tv, keys, vals, n, g, 0u};
   }
 };
@@ -390,16 +392,21 @@ struct RsBatch {
   uint64_t n[kRsBatchMax];
   uint32_t start[kRsBatchMax + 1];
   uint32_t count;
-  __device__ __forceinline__ RsGroup<K, P> group(unsigned int g) const {
+  static constexpr bool kMany = true;
+  // the array that owns group g
+  __device__ __forceinline__ unsigned int find(unsigned int g) const {
     int lo = 0, hi = (int)count - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (start[mid] <= g) lo = mid;
       else hi = mid - 1;
     }
-    return RsGroup<K, P>{keys[lo], vals[lo], tk[lo], tv[lo], src_k[lo], src_v[lo], n[lo], g - start[lo],
-                         (uint32_t)lo};
+    return (unsigned int)lo;
   }
+  __device__ __forceinline__ RsGroup<K, P> group(unsigned int g, unsigned int a) const {
+    return RsGroup<K, P>{keys[a], vals[a], tk[a], tv[a], src_k[a], src_v[a], n[a], g - start[a], a};
+  }
+  __device__ __forceinline__ RsGroup<K, P> group(unsigned int g) const { return group(g, find(g)); }
 };
 
 // Elements of tile `rank` of group `g` (0 past the array's end) and where it starts.
@@ -750,9 +757,9 @@ constexpr size_t rs_smem_bytes() {
 // its tile's keys of those digits.  A lane has DPC / 32 digits.
 template <typename Src, int C, typename K, typename P>
 __device__ __forceinline__ void rs_scout(const Src &src, int pass, unsigned int groups, unsigned int g,
-                                         const unsigned int *hist, unsigned int *status, unsigned int *status_next,
+                                         unsigned int array, const unsigned int *hist, unsigned int *status, unsigned int *status_next,
                                          WsHeader *hdr, unsigned long long limit_ns, const unsigned int *s_x,
-                                         unsigned int *s_base, const unsigned int *s_next, uint64_t *cnt_bar,
+                                         unsigned int *s_base, const uint2 *s_next, uint64_t *cnt_bar,
                                          uint64_t *base_bar) {
   constexpr int DPC = kRsBins / C, DPL = DPC / 32;
   constexpr int WINDOW = kRsWindow / DPL;
@@ -764,7 +771,7 @@ __device__ __forceinline__ void rs_scout(const Src &src, int pass, unsigned int 
       if (lane == 0) record_error(hdr, BK_ERR_SPIN_TIMEOUT, g);
       return;
     }
-    const RsGroup<K, P> gr = src.group(g);
+    const RsGroup<K, P> gr = src.group(g, array);
     const unsigned int *xs = s_x + par * kRsBins + lane;
     unsigned int *row = status + (uint64_t)g * kRsBins + me * DPC + lane;
     unsigned int x[C][DPL], total[DPL], excl[DPL];
@@ -852,7 +859,8 @@ __device__ __forceinline__ void rs_scout(const Src &src, int pass, unsigned int 
       }
       status_next[(uint64_t)g * kRsBins + me * DPC + 32 * e + lane] = 0u;
     }
-    g = s_next[par];
+    g = s_next[par].x;
+    array = s_next[par].y;
   }
 }
 
@@ -863,7 +871,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   using Cfg = RsCfg<K, P>;
   constexpr int ITEMS = Cfg::ITEMS, WARPS = Cfg::WARPS, THREADS = Cfg::THREADS, TILE = Cfg::TILE;
   constexpr int DPC = kRsBins / C;  // digits whose positions this CTA works out
-  constexpr uint32_t COUNT_TX = kRsBins * 4 + 4, BASE_TX = kRsBins * 4;
+  constexpr uint32_t GROUP_TX = Src::kMany ? 8 : 4, COUNT_TX = kRsBins * 4 + GROUP_TX, BASE_TX = kRsBins * 4;
   extern __shared__ __align__(16) unsigned char smem[];
   K *sk = reinterpret_cast<K *>(smem);  // the tile in digit order
   P *sv = reinterpret_cast<P *>(smem + align_up(sizeof(K) * TILE, 16));
@@ -873,11 +881,11 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   // what the peers send, by the iteration's parity (a peer may be one iteration ahead):
   __shared__ unsigned int s_x[2][C][DPC];      // the cluster's counts of this CTA's digits
   __shared__ unsigned int s_base[2][kRsBins];  // output position of the tile's first key of a digit
-  __shared__ unsigned int s_next[2];           // the next iteration's group
+  __shared__ uint2 s_next[2];                  // the next iteration's group and its array
   __shared__ __align__(8) uint64_t s_cnt_bar[2], s_base_bar[2];  // counts and a group, positions are in
   __shared__ unsigned int s_dst[kRsBins];   // output position of staged position 0 for digit d
   __shared__ unsigned int s_scan[kRsBins / 32];
-  __shared__ unsigned int s_group;           // the first group
+  __shared__ uint2 s_group;                  // the first group
   __shared__ __align__(8) uint64_t s_group_bar;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned int me = rs_cluster_rank();
@@ -898,7 +906,8 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
     }
     mbar_init(&s_group_bar, 1);
     rs_fence_mbar_init();
-    mbar_arrive_expect_tx(&s_group_bar, 4);
+    mbar_arrive_expect_tx(&s_group_bar, GROUP_TX);
+    s_group.y = s_next[0].y = s_next[1].y = 0u;
   }
   rs_cluster_sync();  // every CTA of the cluster runs, its barriers ready, before anything is sent to it
   grid_dependency_wait();
@@ -924,31 +933,38 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
   // whoever starts first.
   const unsigned int clusters = gridDim.x / C;
   const bool more = groups > clusters;
+  // the cluster's first warp gives every CTA group t and the array that owns
+  // it (found here once, not by every thread that needs it)
+  auto hand_out = [&](unsigned int t, uint2 *to, const uint64_t *bar) {
+    if (lane < C) {
+      rs_push_u32(&to->x, t, bar, (uint32_t)lane);
+      if constexpr (Src::kMany) rs_push_u32(&to->y, src.find(t), bar, (uint32_t)lane);
+    }
+  };
   if (me == 0 && warp == 0) {
     unsigned int t = 0;
     if (lane == 0) t = atomicAdd(&tickets[launch], 1u);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (lane < C) rs_push_u32(&s_group, t, &s_group_bar, (uint32_t)lane);
+    hand_out(__shfl_sync(0xffffffffu, t, 0), &s_group, &s_group_bar);
   }
   bool failed = !rs_wait_cluster(&s_group_bar, 0, limit_ns);
   failed = __syncthreads_or(failed);
-  unsigned int g = failed ? groups : s_group;
+  unsigned int g = failed ? groups : s_group.x, array = s_group.y;
   if (warp == WARPS) {
-    rs_scout<Src, C, K, P>(src, pass, groups, g, hist, status, status_next, hdr, limit_ns, &s_x[0][0][0], &s_base[0][0],
+    rs_scout<Src, C, K, P>(src, pass, groups, g, array, hist, status, status_next, hdr, limit_ns, &s_x[0][0][0], &s_base[0][0],
                            s_next, s_cnt_bar, s_base_bar);
     rs_cluster_sync();
     return;
   }
-  if (g < groups) load_keys(src.group(g));
+  if (g < groups) load_keys(src.group(g, array));
 
   // the tile before this iteration's, staged and waiting for its positions
-  unsigned int prev_g = groups, prev_excl = 0;
+  unsigned int prev_g = groups, prev_array = 0, prev_excl = 0;
   for (unsigned int it = 0;; ++it) {
     const bool cur = g < groups, prev = prev_g < groups;  // the same in every CTA of the cluster
     if (!cur && !prev) break;
     const uint32_t par = it & 1u, phase = (it >> 1) & 1u;
     uint16_t(*whist)[kRsBins] = s_whist[par];
-    const RsGroup<K, P> gr = src.group(cur ? g : prev_g);
+    const RsGroup<K, P> gr = cur ? src.group(g, array) : src.group(prev_g, prev_array);
     const uint64_t tbase = ((uint64_t)gr.local * C + me) * TILE;
     const int count = rs_tile_count(gr, tbase);
     uint32_t dig4[ITEMS / 4];
@@ -1008,8 +1024,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
         rs_push_u32(&s_x[par][me][tid % DPC], cnt, &s_cnt_bar[par], (uint32_t)(tid / DPC));
       }
       if (me == 0 && warp == 0) {
-        ticket = __shfl_sync(0xffffffffu, ticket, 0);
-        if (lane < C) rs_push_u32(&s_next[par], ticket, &s_cnt_bar[par], (uint32_t)lane);
+        hand_out(__shfl_sync(0xffffffffu, ticket, 0), &s_next[par], &s_cnt_bar[par]);
       }
       // payloads on their way
       if constexpr (has_payload<P>()) {
@@ -1033,7 +1048,7 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
     if (failed) break;
     if (prev) {
       // ---- the tile before is written out: staged position p goes to s_dst[digit] + p
-      const RsGroup<K, P> pg = src.group(prev_g);
+      const RsGroup<K, P> pg = src.group(prev_g, prev_array);
       const int pcount = rs_tile_count(pg, ((uint64_t)pg.local * C + me) * TILE);
       K *out_k = odd ? pg.keys : pg.tk;
       P *out_v = odd ? pg.vals : pg.tv;
@@ -1070,8 +1085,10 @@ __global__ void __launch_bounds__((RsCfg<K, P>::CTA_THREADS), (RsCfg<K, P>::MIN_
     }
     prev_g = g;
     prev_excl = tile_excl;
-    g = s_next[par];
-    if (g < groups) load_keys(src.group(g));
+    prev_array = array;
+    g = s_next[par].x;
+    array = s_next[par].y;
+    if (g < groups) load_keys(src.group(g, array));
   }
   if (failed && tid == 0) record_error(hdr, BK_ERR_SPIN_TIMEOUT, g);
   rs_cluster_sync();  // nothing is sent to a CTA that has left

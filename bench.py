@@ -498,10 +498,12 @@ def other_ops(device, peak, quick=False, shift=0):
         ms = _time_op(lambda: bulk_b200.stable_sort_by_key(k, v), prep=prep, reps=reps)
         ksz = k0.element_size()
         byts = 2 * n * (ksz + 4)
-        # LSD radix: the keys are read once for every pass's digit counts, then
-        # each pass (one per key byte) reads and writes keys and payloads
-        passes = ksz
-        moved = n * ksz + passes * 2 * n * (ksz + 4)
+        # LSD radix: the keys are read once for the passes' digit counts, then
+        # each of four passes reads and writes keys and payloads; 8-byte keys
+        # (uniform: sorted by their upper digits) are read once more for the
+        # runs that agree there
+        passes = 4
+        moved = n * ksz * (2 if ksz == 8 else 1) + passes * 2 * n * (ksz + 4)
         res[f"sort_by_key_{tag}_u32_2^{26 - shift}"] = {
             "ms": ms, "GBps": byts / ms / 1e6, "frac_of_hbm": byts / ms / 1e6 / peak, "algorithmic_bytes": byts,
             "radix_passes": passes,

@@ -1447,7 +1447,7 @@ int radix_sort_launch(K *keys, P *vals, uint64_t n, void *d_ws, size_t ws_bytes,
   }
   if (n >= kRsMaxN) return BK_ERR_TOO_LARGE;  // the caller sorts these by merging
   const RsLayout<K, P> L(&n, 1);
-  if ((st = host::check_ws(d_ws, ws_bytes, L.total)) != BK_OK) return st;
+  if ((st = host::check_ws(d_ws, ws_bytes, L.hist)) != BK_OK) return st;  // the temporaries: all a cluster needs
   char *ws = reinterpret_cast<char *>(d_ws);
   K *tk = reinterpret_cast<K *>(ws + L.tmp);
   P *tv = reinterpret_cast<P *>(ws + L.tmp + align_up(n * sizeof(K), 256));
@@ -1464,6 +1464,7 @@ int radix_sort_launch(K *keys, P *vals, uint64_t n, void *d_ws, size_t ws_bytes,
   if ((st = cluster(integral_constant<int, 512>(), integral_constant<int, 4>())) != kNoCluster) return st;
   if ((st = cluster(integral_constant<int, 1024>(), integral_constant<int, 4>())) != kNoCluster) return st;
   if ((st = cluster(integral_constant<int, 1024>(), integral_constant<int, 8>())) != kNoCluster) return st;
+  if ((st = host::check_ws(d_ws, ws_bytes, L.total)) != BK_OK) return st;
   return radix_sort_run<K, P, RsOne<K, P>, kRsCtas>(RsOne<K, P>{keys, vals, tk, tv, n}, L, ws, stream);
 }
 

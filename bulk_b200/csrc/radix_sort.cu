@@ -443,9 +443,9 @@ constexpr int kRsSampleThreads = 512, kRsSampleCtas = 32, kRsSamples = kRsSample
 constexpr int kRsSampleSlots = 65536;
 constexpr uint32_t kRsSampleWindow = 65536;   // keys a CTA samples from
 // From here on arrays are planned.  u64/u32 on a B200, planned / all eight
-// passes: random keys 2^20 128 / 128 us, 2^22 218 / 300, 2^25 1060 / 1801,
-// 2^26 2009 / 3500; keys of 1000 values (the plan is all passes, and the idle
-// launches are lost) 2^20 159 / 118, 2^22 292 / 250, 2^25 1576 / 1533.
+// passes: random keys 2^20 95 / 111 us, 2^22 186 / 269, 2^25 1020 / 1772, 2^26
+// 1970 / 3500; keys of 1000 values (the plan is all passes, and the idle
+// launches are lost) 2^20 123 / 96, 2^22 254 / 224, 2^25 1536 / 1499.
 constexpr uint64_t kRsPlanMinN = 1ull << 22;
 
 // A key's run has on average 1 + n * sum(p^2) keys (p the shares of the upper

@@ -443,9 +443,11 @@ constexpr int kRsSampleThreads = 512, kRsSampleCtas = 32, kRsSamples = kRsSample
 constexpr int kRsSampleSlots = 65536;
 constexpr uint32_t kRsSampleWindow = 65536;   // keys a CTA samples from
 // From here on arrays are planned.  u64/u32 on a B200, planned / all eight
-// passes: random keys 2^20 95 / 111 us, 2^22 186 / 269, 2^25 1020 / 1772, 2^26
-// 1970 / 3500; keys of 1000 values (the plan is all passes, and the idle
-// launches are lost) 2^20 123 / 96, 2^22 254 / 224, 2^25 1536 / 1499.
+// passes: random keys 2^20 95 / 111 us, 2^22 183 / 269, 2^25 1018 / 1767, 2^26
+// 1967 / 3457; keys of 1000 values (the plan is all passes, and the idle
+// launches are lost) 2^20 123 / 96, 2^22 252 / 224, 2^25 1533 / 1499, 2^26
+// 2956 / 2921.  f64 uniform in [-1, 1): 2^22 217 / 284, 2^25 1570 / 1912, but
+// 2^26 3821 / 3782, where the plan is all passes.
 constexpr uint64_t kRsPlanMinN = 1ull << 22;
 
 // A key's run has on average 1 + n * sum(p^2) keys (p the shares of the upper

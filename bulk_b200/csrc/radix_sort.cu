@@ -773,6 +773,10 @@ __device__ __forceinline__ void rs_scout(const Src &src, int pass, unsigned int 
       if (lane == 0) record_error(hdr, BK_ERR_SPIN_TIMEOUT, g);
       return;
     }
+    // Read before any position is sent: the positions let the cluster's first
+    // CTA run on to the iteration after next, whose group it hands out in the
+    // same place.
+    const uint2 next = s_next[par];
     const RsGroup<K, P> gr = src.group(g, array);
     const unsigned int *xs = s_x + par * kRsBins + lane;
     unsigned int *row = status + (uint64_t)g * kRsBins + me * DPC + lane;
@@ -861,8 +865,8 @@ __device__ __forceinline__ void rs_scout(const Src &src, int pass, unsigned int 
       }
       status_next[(uint64_t)g * kRsBins + me * DPC + 32 * e + lane] = 0u;
     }
-    g = s_next[par].x;
-    array = s_next[par].y;
+    g = next.x;
+    array = next.y;
   }
 }
 

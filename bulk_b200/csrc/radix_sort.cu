@@ -519,15 +519,17 @@ __global__ void __launch_bounds__(kRsSampleThreads) rs_sample_kernel(const K *ke
 // within a run) by the lower halves, in place.  A warp sorts the runs that
 // start in its chunk of keys, which may reach into the kRsFixHalo keys after
 // it; the warp there sees that its first keys belong to an earlier run (their
-// upper halves do not change) and leaves them alone.  A key's place in its
-// run is the number of keys before it with a lower half not above its own
-// plus the number after it with one below: runs are a few keys long, and a
-// key without equal neighbours costs two comparisons.  A run longer than
+// upper halves do not change) and leaves those in the halo alone.  A key's
+// place in its run is the number of keys before it with a lower half not above
+// its own plus the number after it with one below: runs are a few keys long,
+// and a key without equal neighbours costs two comparisons.  A run longer than
 // kRsFixHalo is left as it is, and unless it is in order already (one value
-// many times) the array is sent to the rescue passes.  One read of the keys,
-// bound by memory where runs are rare; warps work on their own, so that one
-// warp's loads run behind another's comparisons (a CTA-wide tile of 4096 keys
-// between barriers took 271 us for 2^26 random keys on a B200).
+// many times) the array is sent to the rescue passes: each of its keys is
+// compared with the one before, by the warp before for a chunk's first
+// kRsFixHalo keys and by the chunk's own warp from the next on.  One read of
+// the keys, bound by memory where runs are rare; warps work on their own, so
+// that one warp's loads run behind another's comparisons (a CTA-wide tile of
+// 4096 keys between barriers took 271 us for 2^26 random keys on a B200).
 constexpr int kRsFixThreads = 128, kRsFixPer = 8, kRsFixChunk = 32 * kRsFixPer, kRsFixHalo = 64;
 
 template <typename K, typename P>
@@ -547,7 +549,6 @@ __global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *v
   const uint64_t step = (uint64_t)gridDim.x * WARPS * kRsFixChunk;
   for (uint64_t base = ((uint64_t)blockIdx.x * WARPS + warp) * kRsFixChunk; base < n; base += step) {
     const int len = (int)((n - base) < (uint64_t)LEN ? (n - base) : (uint64_t)LEN);
-    const bool open = base + (uint64_t)len < n;  // keys follow the halo
     K *const kp = keys + base;
     {
       K k[PER];
@@ -584,13 +585,14 @@ __global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *v
         --first;
         rank += low[first] <= l;
       }
-      // another warp's: it begins before the chunk, or in the halo
-      if ((first == 0 && up[-1] == u) || first >= kRsFixChunk) continue;
+      // another warp's: the run begins before the chunk and the key lies in the
+      // halo of the warp before, or it begins in the halo
+      if ((first == 0 && up[-1] == u && i < kRsFixHalo) || first >= kRsFixChunk) continue;
       while (last - first < kRsFixHalo && last + 1 < len && up[last + 1] == u) {
         ++last;
         rank += low[last] < l;
       }
-      if (last - first >= kRsFixHalo || (open && last + 1 == len)) {
+      if (last - first >= kRsFixHalo) {  // (true of a run that reaches the halo's end)
         if (i > first && low[i - 1] > l) plan->rescue = 1u;
       } else if (first + rank != i) {
         s_to[warp][i] = (uint16_t)(first + rank);

@@ -6,9 +6,9 @@
 // merge.cu:12-97), which is keys-only; the by-key form follows the bounded
 // group merge_by_key (bulk/algorithm/merge.hpp:507-607).
 //
-// Here: persistent CTAs merge runs of 4096-output tiles (2048 for 8-byte keys)
-// in a two-buffer pipeline.  A tile's A/B split comes from a partition kernel
-// where a CTA has many tiles, and from the CTA's loader warp otherwise.  The
+// Here: persistent CTAs merge 4096-output tiles (2048 for 8-byte keys) in a
+// two-buffer pipeline.  A tile's A/B split comes from a partition kernel where
+// a CTA has many tiles, and from the CTA's loader warp otherwise.  The
 // loader's first lane brings a tile's A and B key and payload ranges into
 // shared memory with untiled bulk (TMA) copies -- each range widened to whole
 // 16-byte chunks, the ragged ends by plain loads -- while the compute warps
@@ -18,7 +18,8 @@
 // and, once every thread has read its inputs, writes them back in place in the
 // 128-byte-swizzled layout; the loader then stores the tile with tiled tensor
 // copies, which undo the swizzle.  No thread loads or stores a tile element
-// itself on this path.
+// itself on this path.  Inputs that bulk copies cannot bring (an array off the
+// 16-byte boundaries) are copied by the compute warps, in a kernel of its own.
 #include <algorithm>
 
 #include "bk_common.cuh"
@@ -30,7 +31,7 @@ namespace bk {
 
 constexpr int kMergeWarps = 8;                       // compute warps
 constexpr int kMergeCompute = 32 * kMergeWarps;      // compute threads
-constexpr int kMergeThreads = kMergeCompute + 32;    // + the loader warp (one lane works)
+constexpr int kMergeThreads = kMergeCompute + 32;    // + the loader warp
 constexpr int kMergeBufs = 2;
 
 template <typename K, typename P>
@@ -123,10 +124,10 @@ struct MergeArgs {
   uint64_t nb;
   K *out;
   P *outv;
-  const uint64_t *parts;  // the split at every tile boundary, or null: the loader warp finds them
+  const uint64_t *parts;  // PARTS: the split at every tile boundary
   uint64_t tiles;
   uint64_t covered_out;  // leading outputs inside whole rows of both output views (0: none)
-  int tma_in;            // a, b, av, bv 16-byte aligned: inputs arrive by bulk copies
+  int strided;            // PARTS: CTA c takes tiles c, c + G, c + 2G, ... (G = gridDim.x) instead of a run
 };
 
 // Bytes of the bulk copy that merge_load_range issues for [lo, hi).
@@ -151,15 +152,19 @@ __device__ __forceinline__ void merge_load_range(T *dst, const T *src, uint64_t 
 }
 
 // Persistent merge.  Warps 0-7 merge; warp 8's lane 0 loads and stores.
-// CTA c takes the c-th of gridDim.x equal runs of consecutive tiles.  Where a
-// tile's inputs begin (its split) comes from a partition kernel or, with few
-// tiles a CTA, from the loader warp itself, two tiles ahead: a tile's split
-// lies within a tile of the one before, so its search reads what is loaded
-// next anyway and runs while the compute warps merge.  (The partition kernel,
-// one thread a split, waits for 21 to 26 reads one after another: 14 us before
-// a merge of 3.7 million i32 keys that takes 12.)  A warp of its own for the
-// searches made the kernel's registers spill: 447 us for 2 x 2^26 f32/u32
-// pairs against 408.  Tile i of the CTA uses buffer i mod 2 and goes through:
+// Where a tile's inputs begin (its split) comes from a partition kernel
+// (PARTS) or, with few tiles a CTA, from the loader warp itself, two tiles
+// ahead: CTA c then takes the c-th of gridDim.x equal runs of consecutive
+// tiles, a tile's split lies within a tile of the one before, so its search
+// reads what is loaded next anyway and runs while the compute warps merge.
+// (The partition kernel, one thread a split, waits for 21 to 26 reads one after
+// another: 14 us before a merge of 3.7 million i32 keys that takes 12.)  A warp
+// of its own for the searches made the kernel's registers spill: 447 us for
+// 2 x 2^26 f32/u32 pairs against 408.  Kernels of their own for either source
+// of splits (PARTS needs one loader lane alone) and for unaligned inputs
+// (!TMA_IN) leave each the registers the others would take: in one kernel f64
+// 2 x 2^26 took 481 us against 461 here, f64/u32 7 + 9 million 91 against 82.
+// Tile i of the CTA uses buffer i mod 2 and goes through:
 //   loader: (once the compute warps have written tile i-2's outputs to the
 //           buffer and that tile's stores have read them) write the tile's
 //           descriptor, bulk-copy its ranges in; full[b] completes;
@@ -171,7 +176,7 @@ __device__ __forceinline__ void merge_load_range(T *dst, const T *src, uint64_t 
 //           compute threads directly).
 // All waits are bounded; after a timeout the kernel records
 // BK_ERR_SPIN_TIMEOUT in the header and every role stops.
-template <typename K, typename P>
+template <typename K, typename P, bool TMA_IN, bool PARTS>
 __global__ void __launch_bounds__(kMergeThreads, (sizeof(K) == 4 && payload_bytes<P>() == 8) ? 2 : 3)
 merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
                                                                  WsHeader *hdr, unsigned long long spin_limit_ns) {
@@ -201,11 +206,14 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
   __syncthreads();
   grid_dependency_wait();
 
-  // tiles of this CTA: first + i for i < mine (the grid is no larger than the tile count)
-  const uint64_t first = args.tiles * blockIdx.x / G, mine = args.tiles * (blockIdx.x + 1) / G - first;
+  // tiles of this CTA: first + i * step for i < mine (the grid is no larger than the tile count)
+  const bool strided = PARTS && args.strided;
+  const uint64_t first = strided ? blockIdx.x : args.tiles * blockIdx.x / G, step = strided ? G : 1;
+  const uint64_t mine = strided ? (args.tiles - blockIdx.x + G - 1) / G : args.tiles * (blockIdx.x + 1) / G - first;
 
   if (warp == kMergeWarps) {
     // ================= the loader (lane 0; the splits: all lanes) =================
+    if (PARTS && lane != 0) return;
     // A elements before tile k, given that `from` lie before a tile no more than `tiles` before it
     auto split = [&](uint64_t k, uint64_t from, uint64_t tiles) -> uint64_t {
       const uint64_t diag = k * TILE < total ? k * TILE : total;
@@ -234,7 +242,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     };
     const uint64_t *const parts = args.parts;
     uint64_t a0, a1;  // the A range of the tile to load next
-    if (parts != nullptr) {
+    if constexpr (PARTS) {
       a0 = parts[first];
       a1 = parts[first + 1];
     } else {
@@ -252,9 +260,9 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
         // tile i-2's outputs are in buffer b: store them
         if (lane == 0 && !mbar_wait_or_abort(&s_out[b], (outpar >> b) & 1u, spin_limit_ns, &s_abort)) {
           failed = true;
-          fail_tile = first + i - 2;
+          fail_tile = first + (i - 2) * step;
         }
-        if (__shfl_sync(0xffffffffu, (int)failed, 0)) break;
+        if (PARTS ? failed : __shfl_sync(0xffffffffu, (int)failed, 0) != 0) break;
         outpar ^= 1u << b;
         const uint32_t tile = s_desc[b].tile;
         if (lane == 0 && args.covered_out > (uint64_t)tile * TILE) {
@@ -266,7 +274,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
       }
       if (i >= mine) continue;
       // ---- tile k: its A range [a0, a1) and B range [b0, b1)
-      const uint64_t k = first + i;
+      const uint64_t k = first + i * step;
       if (lane == 0) {
         if (stored) tma_store_wait_read();  // the stores have read the buffer
         const uint64_t d0 = k * TILE, d1 = d0 + TILE < total ? d0 + TILE : total;
@@ -277,7 +285,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
         d.count = (uint32_t)(d1 - d0);
         d.tile = (uint32_t)k;
         d.a0 = a0;
-        if (args.tma_in) {
+        if constexpr (TMA_IN) {
           const uint64_t alo = a0 & ~(uint64_t)(C::L - 1), blo = b0 & ~(uint64_t)(C::L - 1);
           const uint32_t bstart = (uint32_t)align_up(a1 - alo, (size_t)C::L);  // B's copy: a multiple of L
           d.ia = (uint32_t)(a0 - alo);
@@ -304,14 +312,15 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
         // ends): the phase completes once the bulk copies' bytes have landed
         mbar_arrive(&s_full[b]);
       }
-      __syncwarp();
+      if constexpr (!PARTS) __syncwarp();
       armpar ^= 1u << b;
       armany |= 1u << b;
       if (i + 1 < mine) {  // the next tile's end, while this one is merged
-        a0 = a1;
-        if (parts != nullptr) {
-          a1 = parts[k + 2];
+        if constexpr (PARTS) {
+          a0 = parts[k + step];
+          a1 = parts[k + step + 1];
         } else {
+          a0 = a1;
           a1 = split(k + 2, a0, 1);
           if (lane == 0) prefetch(k + 1, a0, a1);
         }
@@ -334,7 +343,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
   bool bad = false;
   for (uint64_t i = 0; i < mine; ++i) {
     const int b = (int)(i & 1);
-    const uint64_t k = first + i;
+    const uint64_t k = first + i * step;
     if (!mbar_wait_or_abort(&s_full[b], (fullpar >> b) & 1u, spin_limit_ns, &s_abort)) bad = true;
     fullpar ^= 1u << b;
     if (named_barrier_or(1, kMergeCompute, bad || aborted())) {
@@ -345,7 +354,7 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     const MergeDesc d = s_desc[b];
     K *const sk = reinterpret_cast<K *>(buf(b));
     P *const sp = reinterpret_cast<P *>(buf(b) + C::KEY_AREA);
-    if (!args.tma_in) {  // a launch-wide flag: every compute warp takes this branch or none
+    if constexpr (!TMA_IN) {
       const uint64_t a0 = d.a0, b0 = k * TILE - a0;
       for (uint32_t j = tid; j < d.la; j += kMergeCompute) {
         sk[j] = args.a[a0 + j];
@@ -448,6 +457,8 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
   }
 }
 
+constexpr int kOther = 1 << 30;  // no status
+
 template <typename K>
 size_t merge_ws_bytes(uint64_t n) {
   const uint64_t tiles = (n + MergeCfg<K, NoPayload>::TILE - 1) / MergeCfg<K, NoPayload>::TILE;
@@ -488,7 +499,7 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   args.outv = outv;
   args.tiles = tiles;
   auto a16 = [](const void *p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  args.tma_in = a16(a) && a16(b) && a16(av) && a16(bv);
+  const bool tma_in = a16(a) && a16(b) && a16(av) && a16(bv);  // inputs arrive by bulk copies
   // output row views: the outputs inside whole 128-byte rows of both leave by
   // tensor stores, the rest by plain stores
   const uint64_t krows = n * sizeof(K) / 128, prows = n * (uint64_t)C::PB / 128;
@@ -502,13 +513,9 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
     }
   }
   const size_t smem = merge_smem_bytes<K, P>();
-  struct Site {};
-  host::KernelSetup ks;
-  if ((st = host::kernel_setup<Site>(merge_kernel<K, P>, kMergeThreads, smem, &ks)) != BK_OK) return st;
   const tune::Knobs kn = tune::knobs_for(tune::kMerge, (int)(sizeof(K) + C::PB), n);
-  const uint64_t per_sm = ks.resident_ctas / (uint64_t)di.sm_count;  // what fits (shared memory, registers)
-  const uint64_t want = (uint64_t)di.sm_count * (uint64_t)std::max(kn.ctas_per_sm, 1);
-  const unsigned grid = (unsigned)std::min<uint64_t>(tiles, std::min<uint64_t>(want, std::max<uint64_t>(per_sm, 1) * di.sm_count));
+  const host::DebugFault dbg = host::debug_fault();
+  const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
   // Many tiles a CTA: a partition kernel first, whose splits cost the loader
   // nothing; few: the loader finds them (see merge_kernel).  Measured on a
   // B200, partition / loader: f32/u32 2 x 2^18 17.4 / 13.0 us, 2 x 2^22 46.1 /
@@ -517,17 +524,45 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   // 169 / 181; f64 2 x 2^22 52.2 / 47.1, 2 x 2^24 136.2 / 135.2; f32 2 x 2^18
   // 15.3 / 11.1, 2 x 2^26 273 / 262 (keys of 4 bytes alone never need it).
   constexpr uint64_t kPerCta = C::PB == 0 ? (sizeof(K) == 4 ? ~0ull : 16) : (sizeof(K) == 4 ? 16 : 8);
-  if (tiles / kPerCta >= grid) {
-    uint64_t *parts = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(d_ws) + kHeaderBytes);
-    const uint64_t np = tiles + 1;
-    st = host::launch_overlapped(merge_partition_kernel<K>, (unsigned)((np + 255) / 256), 256, 0, stream, 1, a, na, b, nb,
-                                 (uint64_t)C::TILE, np, parts);
-    if (st != BK_OK) return st;
-    args.parts = parts;
-  }
-  const host::DebugFault dbg = host::debug_fault();
-  const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
-  return host::launch_overlapped(merge_kernel<K, P>, grid, kMergeThreads, smem, stream, 1, args, hdr, limit);
+  // With a partition kernel the CTAs' tiles are interleaved, so that all of
+  // them read and write close to one another; 4-byte keys from 32 tiles a CTA
+  // on do better with a run each.  Interleaved / runs: i32/u32 2 x 2^24 (18 a
+  // CTA) 107.5 / 111.6 us, 2 x 2^25 (37) 208.8 / 202.7, 2 x 2^26 403 / 397;
+  // i32/u64 2 x 2^24 (28) 151.6 / 158.7, 2 x 2^25 (55) 293.7 / 286.6; f64/u32
+  // 7 + 9 million 83.9 / 91.1, 2 x 2^25 of few values 280 / 290; f64/u64 60
+  // million + 1000 309 / 328.
+  constexpr uint64_t kRunsFrom = sizeof(K) == 4 ? 32 : ~0ull;
+  auto launch = [&](auto tma, auto parted) -> int {  // kOther when the other source of splits is the better one
+    constexpr bool PARTS = decltype(parted)::value;
+    auto kern = merge_kernel<K, P, decltype(tma)::value, PARTS>;
+    struct Site {};
+    host::KernelSetup ks;
+    int e = host::kernel_setup<Site>(kern, kMergeThreads, smem, &ks);
+    if (e != BK_OK) return e;
+    const uint64_t per_sm = ks.resident_ctas / (uint64_t)di.sm_count;  // what fits (shared memory, registers)
+    const uint64_t want = (uint64_t)di.sm_count * (uint64_t)std::max(kn.ctas_per_sm, 1);
+    const unsigned grid =
+        (unsigned)std::min<uint64_t>(tiles, std::min<uint64_t>(want, std::max<uint64_t>(per_sm, 1) * di.sm_count));
+    if (!PARTS && tiles / kPerCta >= grid) return kOther;
+    if constexpr (PARTS) {
+      uint64_t *parts = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(d_ws) + kHeaderBytes);
+      const uint64_t np = tiles + 1;
+      e = host::launch_overlapped(merge_partition_kernel<K>, (unsigned)((np + 255) / 256), 256, 0, stream, 1, a, na, b, nb,
+                                  (uint64_t)C::TILE, np, parts);
+      if (e != BK_OK) return e;
+      args.parts = parts;
+      args.strided = tiles / kRunsFrom < grid;
+    }
+    return host::launch_overlapped(kern, grid, kMergeThreads, smem, stream, 1, args, hdr, limit);
+  };
+  auto merge = [&](auto tma) -> int {
+    const int e = launch(tma, std::false_type());
+    if constexpr (kPerCta != ~0ull) {
+      if (e == kOther) return launch(tma, std::true_type());
+    }
+    return e;
+  };
+  return tma_in ? merge(std::true_type()) : merge(std::false_type());
 }
 
 size_t merge_workspace_bytes(int key_dtype, int value_dtype, uint64_t n) {

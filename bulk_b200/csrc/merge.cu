@@ -151,6 +151,21 @@ __device__ __forceinline__ void merge_load_range(T *dst, const T *src, uint64_t 
   for (uint64_t i = bulk_hi > lo ? bulk_hi : lo; i < hi; ++i) dst[i - lo] = src[i];
 }
 
+// One element from global to shared memory, with no register in between: the
+// compute warps' copy of inputs that bulk copies cannot bring.  Through
+// registers it was bound by the loads' latency, or by the instructions of
+// loads batched by hand (half as many again, ncu): whether the compiler kept
+// several loads in flight turned on the registers left (i32/u32 2 x 2^26 off
+// the boundaries on a B200: 654 us, and 1029 after unrelated changes; u32/u64
+// 2140).  With all of a tile's copies in flight: 598, 817.
+template <typename T>
+__device__ __forceinline__ void copy_async(T *dst, const T *src) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "4 or 8 bytes");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"((int)sizeof(T)) : "memory");
+}
+// Until this thread's copies have arrived.
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Persistent merge.  Warps 0-7 merge; warp 8's lane 0 loads and stores.
 // Where a tile's inputs begin (its split) comes from a partition kernel
 // (PARTS) or, with few tiles a CTA, from the loader warp itself, two tiles
@@ -357,13 +372,14 @@ merge_kernel(const __grid_constant__ MergeArgs<K, P> args,
     if constexpr (!TMA_IN) {
       const uint64_t a0 = d.a0, b0 = k * TILE - a0;
       for (uint32_t j = tid; j < d.la; j += kMergeCompute) {
-        sk[j] = args.a[a0 + j];
-        if constexpr (HP) sp[j] = args.av[a0 + j];
+        copy_async(sk + j, args.a + a0 + j);
+        if constexpr (HP) copy_async(sp + j, args.av + a0 + j);
       }
       for (uint32_t j = tid; j < d.lb; j += kMergeCompute) {
-        sk[d.la + j] = args.b[b0 + j];
-        if constexpr (HP) sp[d.la + j] = args.bv[b0 + j];
+        copy_async(sk + d.la + j, args.b + b0 + j);
+        if constexpr (HP) copy_async(sp + d.la + j, args.bv + b0 + j);
       }
+      copy_async_wait();
       named_barrier_sync(2, kMergeCompute);
     }
     // ---- merge-path search for this thread's first output, then its outputs

@@ -411,7 +411,9 @@ inline int launch_overlapped(void (*kern)(Params...), unsigned grid, unsigned th
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return from_cuda(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();  // reported here, not by the next launch_status() too
+  return from_cuda(e);
 }
 
 // Opt a kernel into `bytes` of dynamic shared memory and the largest shared

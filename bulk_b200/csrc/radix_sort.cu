@@ -1381,7 +1381,10 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if ((e = host::from_cuda(cudaOccupancyMaxActiveClusters(out, pass_kern, &cfg))) != BK_OK) return e;
+    if ((e = host::from_cuda(cudaOccupancyMaxActiveClusters(out, pass_kern, &cfg))) != BK_OK) {
+      (void)cudaGetLastError();
+      return e;
+    }
     return *out > 0 ? BK_OK : BK_ERR_UNSUPPORTED;
   });
   if (st != BK_OK) return st;

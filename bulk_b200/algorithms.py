@@ -142,9 +142,15 @@ def debug_set_fault(skip_publish_tile: int = -1, spin_limit_ns: int = 0) -> None
     check(lib.bk_debug_set_fault(skip_publish_tile, spin_limit_ns), "bk_debug_set_fault")
 
 
-# The workspace a call needs depends on its types and length alone: kept for
-# the lengths in use, so that a repeated call asks the library once.
-_need_bytes = lru_cache(maxsize=4096)(workspace_bytes)
+@lru_cache(maxsize=4096)
+def _need_bytes(device: int, algo: str, key: str, value: str | None, n: int) -> int:
+    """The workspace a call on ``device`` needs.  It depends on types, length
+    and device (the reduce's partials: on its SMs) alone: kept for the lengths
+    in use, so that a repeated call asks the library once."""
+    if device == torch.cuda.current_device():
+        return workspace_bytes(algo, key, value, n)
+    with torch.cuda.device(device):
+        return workspace_bytes(algo, key, value, n)
 
 
 @lru_cache(maxsize=None)
@@ -165,8 +171,8 @@ def _call(fn, dev: torch.device, stream: torch.cuda.Stream | None, need: int, *a
         check(status, fn.__name__)
 
 
-def _need(algo: str, key: str, value: str | None, n: int) -> int:
-    need = _need_bytes(algo, key, value, n)
+def _need(dev: torch.device, algo: str, key: str, value: str | None, n: int) -> int:
+    need = _need_bytes(dev.index, algo, key, value, n)
     return max(need, 256) if need or algo == "reduce" else 0
 
 
@@ -179,7 +185,8 @@ def reduce(x: torch.Tensor, init=0, op: str = "sum", out: torch.Tensor | None = 
     if out is None:
         out = torch.empty(1, dtype=x.dtype, device=dev)
     n = x.numel()
-    _call(_entry("reduce", op, tag), dev, stream, _need("reduce", tag, None, n), x.data_ptr(), n, init, out.data_ptr())
+    need = _need(dev, "reduce", tag, None, n)
+    _call(_entry("reduce", op, tag), dev, stream, need, x.data_ptr(), n, init, out.data_ptr())
     return out
 
 
@@ -199,7 +206,7 @@ def inclusive_scan(x: torch.Tensor, init=0, op: str = "sum", out: torch.Tensor |
         if not init.is_cuda or init.device != dev or init.dtype != x.dtype or init.numel() != 1:
             raise ValueError("a tensor init must be one element of x's dtype on x's device")
     n = x.numel()
-    need = _need("inclusive_scan", tag, None, n)
+    need = _need(dev, "inclusive_scan", tag, None, n)
     if dinit:
         _call(_entry("inclusive_scan", op, tag, "dinit"), dev, stream, need, x.data_ptr(), n, init.data_ptr(),
               out.data_ptr())
@@ -234,7 +241,7 @@ def merge(a: torch.Tensor, b: torch.Tensor, a_vals: torch.Tensor | None = None, 
     if a_vals is not None and out_vals is None:
         out_vals = torch.empty(n, dtype=a_vals.dtype, device=dev)
     vt = _payload_tag(a_vals)
-    need = _need("merge", tag, vt, n)
+    need = _need(dev, "merge", tag, vt, n)
     if a_vals is None:
         _call(_entry("merge", tag), dev, stream, need, a.data_ptr(), a.numel(), b.data_ptr(), b.numel(), out.data_ptr())
         return out
@@ -252,7 +259,7 @@ def stable_sort_by_key(keys: torch.Tensor, vals: torch.Tensor | None = None,
     if vals is not None and vals.numel() != n:
         raise ValueError("keys and vals must have the same length")
     vt = _payload_tag(vals)
-    need = _need("sort_by_key", tag, vt, n)
+    need = _need(dev, "sort_by_key", tag, vt, n)
     if vals is None:
         _call(_entry("sort_keys", tag), dev, stream, need, keys.data_ptr(), n)
         return keys
@@ -281,7 +288,7 @@ def reduce_by_key(keys: torch.Tensor, vals: torch.Tensor, out_keys: torch.Tensor
         out_vals = torch.empty(max(n, 1), dtype=vals.dtype, device=dev)
     if num_out is None:
         num_out = torch.empty(1, dtype=torch.int64, device=dev)
-    _call(_entry("reduce_by_key", kt, vt), dev, stream, _need("reduce_by_key", kt, vt, n), keys.data_ptr(),
+    _call(_entry("reduce_by_key", kt, vt), dev, stream, _need(dev, "reduce_by_key", kt, vt, n), keys.data_ptr(),
           vals.data_ptr(), n, out_keys.data_ptr(), out_vals.data_ptr(), num_out.data_ptr())
     if not sync:
         return out_keys, out_vals, num_out

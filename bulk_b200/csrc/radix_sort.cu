@@ -1498,12 +1498,22 @@ struct RsItem {
 // and a CTA sees all keys: passes whose digit is the same in every key are
 // left out, and 8-byte keys whose upper halves mostly differ are sorted by
 // their upper digits, then their short runs of equal upper halves are put in
-// order in place (by counting, as rs_fix_kernel does).  On a B200, with the
-// block sort by merging before: u32/u32 1024 keys 5.6 us (22.5), 4096 11.8 (24.4);
-// u64/u32 1024 6.2 (18.4), 4096 15.9 (20.0; 22 where few upper halves and all
-// digits occur, so that all eight passes are needed).
+// order in place (by counting, as rs_fix_kernel does).  The keys are counted
+// by a hash of their upper half first, which bounds the runs: a slot holds at
+// least the run's keys, and the sum of the slots' squares at least the
+// comparisons.  (A guess from a sample of the keys met runs of hundreds: 4096
+// u64/u32 keys of which 70 agree took 52 us.)  Runs of up to 64 keys, six on
+// average, cost less than the four lower passes (4096 u64/u32 of 1000 upper
+// halves 20.2 us, by all digits 21.5; of 70 equal ones 28 against 22).
+// 512 threads of eight keys where 1024 of four left each 64 registers and 32
+// warps' counters to sum (u64/u32 4096 random 15.7 us, now 14.1; all digits
+// 24.0, now 21.0).  On a B200, with the block sort by merging before: u32/u32
+// 1024 keys 5.0 us (22.7), 4096 11.0 (24.7); u64/u32 1024 6.3 (18.6), 4096
+// 14.1 (20.9; 22.1 where more than 64 keys share an upper half and all digits
+// occur).
 // ---------------------------------------------------------------------------
-constexpr int kRsBlockMax = 4096, kRsBlockItems = 4;
+constexpr int kRsBlockMax = 4096;
+constexpr unsigned int kRsBlockRun = 64, kRsBlockRunMean = 6;
 
 template <typename K, typename P, int N>
 struct RsBlockItems {
@@ -1514,19 +1524,20 @@ struct RsBlockItems {
   uint32_t n[N];
 };
 
-template <typename K, typename P, int TH>
+template <typename K, typename P, int TH, int ITEMS>
 constexpr size_t rs_block_smem_bytes() {
-  constexpr size_t tile = (size_t)TH * kRsBlockItems;
+  constexpr size_t tile = (size_t)TH * ITEMS;
   return 256 + (size_t)(TH / 32) * (512 + 128) + align_up(sizeof(K) * tile, 16) + (size_t)payload_bytes<P>() * tile;
 }
 
-template <typename K, typename P, int TH, int N>
+template <typename K, typename P, int TH, int ITEMS, int N>
 __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__ RsBlockItems<K, P, N> items) {
-  constexpr int ITEMS = kRsBlockItems, WARPS = TH / 32, TILE = TH * ITEMS;
+  constexpr int WARPS = TH / 32, TILE = TH * ITEMS;
   extern __shared__ __align__(16) unsigned char rs_bl_smem[];
   __shared__ __align__(16) uint16_t s_whist[WARPS][kRsBins];  // per-warp digit counters, then staging starts (both x4)
   __shared__ unsigned int s_scan[kRsBins / 32];
   __shared__ unsigned int s_vary[2];  // bits that differ between keys: lower and upper halves
+  __shared__ unsigned int s_run[2];   // the most keys in a slot, and the sum of the slots' squares
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned char *tables = rs_bl_smem + (256u - (smem_addr(rs_bl_smem) & 255u));
   unsigned char *bits = tables + WARPS * 512;
@@ -1535,13 +1546,22 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
   const RsRanker ranker(tables + warp * 512, bits + warp * 128);
   uint4 *const mine = reinterpret_cast<uint4 *>(&s_whist[warp][0]) + lane;  // a warp clears its own counters
   *mine = make_uint4(0u, 0u, 0u, 0u);
-  if (tid < 2) s_vary[tid] = 0u;
+  // 8-byte keys are counted by a hash of their upper half, in the staging area
+  unsigned int *const slots = reinterpret_cast<unsigned int *>(sk);
+  if constexpr (sizeof(K) == 8) {
+#pragma unroll
+    for (int j = 0; j < ITEMS / 2; ++j) reinterpret_cast<uint4 *>(slots)[j * TH + tid] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (tid < 2) s_vary[tid] = s_run[tid] = 0u;
   __syncthreads();
   grid_dependency_wait();
   const K *in_k = items.in_k[blockIdx.x];
   const P *in_v = items.in_v[blockIdx.x];
   const int count = (int)items.n[blockIdx.x];
   auto elem = [&](int j) { return warp * 32 * ITEMS + j * 32 + lane; };
+  auto slot_of = [&](K key) {
+    return slots + ((unsigned int)rs_word(RadixKey<K>::to(key), 4) * 0x9e3779b1u) / (0x80000000u / (unsigned int)TILE);
+  };
   K k[ITEMS];
   P v[ITEMS];
 #pragma unroll
@@ -1555,8 +1575,12 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
     const auto first = RadixKey<K>::to(in_k[0]);
     typename RadixKey<K>::U x = 0;
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j)
-      if (elem(j) < count) x |= RadixKey<K>::to(k[j]) ^ first;
+    for (int j = 0; j < ITEMS; ++j) {
+      if (elem(j) < count) {
+        x |= RadixKey<K>::to(k[j]) ^ first;
+        if constexpr (sizeof(K) == 8) atomicAdd(slot_of(k[j]), 1u);
+      }
+    }
 #pragma unroll
     for (int h = 0; h < (int)sizeof(K) / 4; ++h) {
       const unsigned int o = __reduce_or_sync(0xffffffffu, rs_word(x, 4 * h));
@@ -1569,43 +1593,59 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
     todo = digits(s_vary[0]);
     if constexpr (sizeof(K) == 8) todo |= digits(s_vary[1]) << 4;
   }
-  const unsigned int all = todo;
-  bool upper = false;  // the upper digits alone, to begin with
+  bool upper = false;  // the upper digits alone, then the runs that agree there
   if constexpr (sizeof(K) == 8) {
-    // not where half of the warps see an upper half twice among 32 keys
-    const bool twice = __popc(__match_any_sync(0xffffffffu, rs_word(RadixKey<K>::to(k[0]), 4))) > 1 && elem(0) < count;
-    const bool warp_twice = __any_sync(0xffffffffu, twice);
-    const int warps = __syncthreads_count(lane == 0 && warp_twice);
-    upper = (all >> 4) != 0u && (all & 15u) != 0u && 2 * warps < (count + 127) / 128;
+    unsigned int most = 0, sum = 0;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      if (elem(j) < count) {
+        const unsigned int c = *slot_of(k[j]);
+        most = c > most ? c : most;
+        sum += c;
+      }
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) {
+      atomicMax(&s_run[0], most);
+      atomicAdd(&s_run[1], sum);
+    }
+    __syncthreads();
+    upper = (todo >> 4) != 0u && (todo & 15u) != 0u && s_run[0] <= kRsBlockRun &&
+            s_run[1] <= kRsBlockRunMean * (unsigned int)count;
   }
   if (upper) todo &= 0xf0u;
   while (todo != 0u) {
     const int pass = __ffs(todo) - 1;
     todo &= todo - 1u;
     // past the array's end the digit is 255: those items stay last
-    uint32_t dig4[1] = {rs_digits4(k, pass)};
+    uint32_t dig4[ITEMS / 4];
+#pragma unroll
+    for (int i = 0; i < ITEMS / 4; ++i) dig4[i] = rs_digits4(k + 4 * i, pass);
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j)
-      if (elem(j) >= count) dig4[0] |= 0xffu << (8 * j);
+      if (elem(j) >= count) dig4[j >> 2] |= 0xffu << (8 * (j & 3));
     uint32_t rank2[ITEMS / 2];
     ranker.rank<ITEMS>(s_whist[warp], dig4, rank2);
     __syncthreads();
     if (tid < kRsBins) {
-      unsigned int cnt = 0, total;
+      unsigned int c[WARPS], cnt = 0, total;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) cnt += s_whist[w][tid];
+      for (int w = 0; w < WARPS; ++w) {
+        c[w] = s_whist[w][tid];
+        cnt += c[w];
+      }
       unsigned int run = rs_scan_digits(cnt, s_scan, total);
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) {
-        const unsigned int c = s_whist[w][tid];
         s_whist[w][tid] = (uint16_t)run;
-        run += c;
+        run += c[w];
       }
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-      const uint32_t d = (dig4[0] >> (8 * j)) & 0xffu;
+      const uint32_t d = (dig4[j >> 2] >> (8 * (j & 3))) & 0xffu;
       const uint32_t pos = (s_whist[warp][d] + ((rank2[j >> 1] >> (16 * (j & 1))) & 0xffffu)) >> 2;
       sk[pos] = k[j];
       if constexpr (has_payload<P>()) sv[pos] = v[j];
@@ -1620,10 +1660,8 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
     }
     if constexpr (sizeof(K) == 8) {
       if (upper && todo == 0u) {
-        upper = false;
-        constexpr int LONGEST = 64;
         int to[ITEMS];
-        bool move = false, redo = false;
+        bool move = false;
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
           const int i = elem(j);
@@ -1631,23 +1669,14 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
           if (i >= count) continue;
           const uint64_t u = RadixKey<K>::to(k[j]);
           auto same = [&](int q) { return (unsigned int)((RadixKey<K>::to(sk[q]) ^ u) >> 32) == 0u; };
-          int first = i, last = i, rank = 0;
-          while (first > 0 && last - first < LONGEST && same(first - 1)) {
-            --first;
-            rank += RadixKey<K>::to(sk[first]) <= u;
-          }
-          while (last + 1 < count && last - first < LONGEST && same(last + 1)) {
-            ++last;
-            rank += RadixKey<K>::to(sk[last]) < u;
-          }
-          if (last - first >= LONGEST) {
-            redo |= i > 0 && same(i - 1) && RadixKey<K>::to(sk[i - 1]) > u;
-          } else if (first + rank != i) {
+          int first = i, rank = 0;
+          for (; first > 0 && same(first - 1); --first) rank += RadixKey<K>::to(sk[first - 1]) <= u;
+          for (int q = i + 1; q < count && same(q); ++q) rank += RadixKey<K>::to(sk[q]) < u;
+          if (first + rank != i) {
             to[j] = first + rank;
             move = true;
           }
         }
-        redo = __syncthreads_or(redo);
         if (__syncthreads_or(move)) {
 #pragma unroll
           for (int j = 0; j < ITEMS; ++j) {
@@ -1663,7 +1692,6 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
             if constexpr (has_payload<P>()) v[j] = sv[elem(j)];
           }
         }
-        if (redo) todo = all;  // a long run out of order: all digits (equal keys are still in input order)
       }
     }
   }
@@ -1676,14 +1704,14 @@ __global__ void __launch_bounds__(TH, 1) rs_block_kernel(const __grid_constant__
   }
 }
 
-template <typename K, typename P, int TH, int N>
+template <typename K, typename P, int TH, int ITEMS, int N>
 int rs_block_run(const RsBlockItems<K, P, N> &items, uint32_t count, cudaStream_t stream) {
   struct Site {};
   host::KernelSetup ks;
-  constexpr size_t smem = rs_block_smem_bytes<K, P, TH>();
-  const int st = host::kernel_setup<Site>(rs_block_kernel<K, P, TH, N>, TH, smem, &ks);
+  constexpr size_t smem = rs_block_smem_bytes<K, P, TH, ITEMS>();
+  const int st = host::kernel_setup<Site>(rs_block_kernel<K, P, TH, ITEMS, N>, TH, smem, &ks);
   if (st != BK_OK) return st;
-  return host::launch_overlapped(rs_block_kernel<K, P, TH, N>, count, TH, smem, stream, 1, items);
+  return host::launch_overlapped(rs_block_kernel<K, P, TH, ITEMS, N>, count, TH, smem, stream, 1, items);
 }
 
 // `count` arrays of 1 to kRsBlockMax keys each, checked by the caller.
@@ -1703,9 +1731,9 @@ int radix_sort_blocks(const RsItem<K, P> *items, uint32_t count, cudaStream_t st
       longest = items[i].n > longest ? items[i].n : longest;
     }
     if (m == 0) return (int)BK_OK;
-    return longest <= 1024   ? rs_block_run<K, P, 256, decltype(cap)::value>(b, m, stream)
-           : longest <= 2048 ? rs_block_run<K, P, 512, decltype(cap)::value>(b, m, stream)
-                             : rs_block_run<K, P, 1024, decltype(cap)::value>(b, m, stream);
+    return longest <= 1024   ? rs_block_run<K, P, 256, 4, decltype(cap)::value>(b, m, stream)
+           : longest <= 2048 ? rs_block_run<K, P, 512, 4, decltype(cap)::value>(b, m, stream)
+                             : rs_block_run<K, P, 512, 8, decltype(cap)::value>(b, m, stream);
   };
   return count == 1 ? run(std::integral_constant<int, 1>()) : run(std::integral_constant<int, kRsBatchMax>());
 }

@@ -426,16 +426,20 @@ __device__ __forceinline__ int rs_tile_count(const RsGroup<K, P> &g, uint64_t ba
 // kernel launched after it works the decision out (a kernel with nothing to
 // do leaves at once):
 //   full    the passes of digits 0-3 and 4-7
-//   upper   the passes of digits 4-7, then rs_fix_kernel
-//   rescue  rs_fix_kernel met a run longer than it sorts (the sample missed
-//           it): the passes of digits 0-3 and 4-7 follow.  The array then
-//           holds its keys in another order, but equal keys still in input
-//           order, so the result is the same.
+//   upper   the passes of digits 4-7, then rs_fix_kernel; where that met runs
+//           longer than it sorts and out of order (the sample missed them),
+//           rs_late_kernel sorts those
+//   rescue  more or longer runs than rs_late_kernel takes: the passes of
+//           digits 0-3 and 4-7 follow.  The array then holds its keys in
+//           another order, but equal keys still in input order, so the result
+//           is the same.
 struct RsPlanWs {
-  unsigned int repeats;  // sampled keys whose upper half another one has
-  unsigned int zeros;    // sampled keys whose upper half is zero
-  unsigned int rescue;
-  unsigned int pad;
+  unsigned int repeats;    // sampled keys whose upper half another one has
+  unsigned int zeros;      // sampled keys whose upper half is zero
+  unsigned int unordered;  // a run that rs_fix_kernel left alone is out of order
+  unsigned int too_many;   // such runs do not fit their list, or one is longer than rs_late_kernel takes
+  unsigned int runs[2];    // listed runs: of up to kRsRunWarp keys, longer
+  unsigned int pad[2];
 };
 enum RsPlan { kPlanFull, kPlanUpper, kPlanRescue };
 
@@ -449,6 +453,26 @@ constexpr uint32_t kRsSampleWindow = 65536;   // keys a CTA samples from
 // 2956 / 2921.  f64 uniform in [-1, 1): 2^22 217 / 284, 2^25 1570 / 1912, but
 // 2^26 3821 / 3782, where the plan is all passes.
 constexpr uint64_t kRsPlanMinN = 1ull << 22;
+// What rs_late_kernel takes: runs of up to kRsRunWarp keys a warp each, of up to
+// kRsRunMax a CTA each.  They are listed in the status rows that the passes
+// between use next (one word in 54 to 72 keys): the longer ones from the end.
+// Without it one such run sent the array to the rescue, whose twelve passes
+// take longer than eight by separate counting and scattering did.  u64/u32 on a
+// B200, random keys and some such runs: those eight 430 us at 2^22 and 4610 at
+// 2^26, rescue 471 and 5408, now, by the runs: one of 400 231 and 2015, one of
+// 60,000 299 (all passes) and 2280, one of 66 keys for each 1000 300 and 2850.
+// (Runs of 1000 by a warp each took 409 us at 2^22, by a CTA 232.)
+constexpr unsigned int kRsRunWarp = 256, kRsRunMax = 131072;
+struct RsRunList {
+  unsigned int *start;  // where each run begins
+  unsigned int room;
+  __device__ __forceinline__ unsigned int room_for(bool longer, uint32_t n) const {
+    return longer ? n / kRsRunWarp : room - n / kRsRunWarp;
+  }
+  __device__ __forceinline__ unsigned int *slot(bool longer, unsigned int i) const {
+    return start + (longer ? room - 1u - i : i);
+  }
+};
 
 // A key's run has on average 1 + n * sum(p^2) keys (p the shares of the upper
 // halves' values), of which the sample's repeats estimate 2 * repeats /
@@ -456,7 +480,7 @@ constexpr uint64_t kRsPlanMinN = 1ull << 22;
 __device__ __forceinline__ RsPlan rs_plan(const RsPlanWs *plan, uint64_t n) {
   if (plan == nullptr) return kPlanFull;
   const uint4 w = ld_cg_v4(plan);
-  if (w.z != 0u) return kPlanRescue;
+  if (w.z != 0u && w.w != 0u) return kPlanRescue;
   return (uint64_t)w.x * n <= 4ull * kRsSamples * kRsSamples ? kPlanUpper : kPlanFull;
 }
 
@@ -523,17 +547,19 @@ __global__ void __launch_bounds__(kRsSampleThreads) rs_sample_kernel(const K *ke
 // place in its run is the number of keys before it with a lower half not above
 // its own plus the number after it with one below: runs are a few keys long,
 // and a key without equal neighbours costs two comparisons.  A run longer than
-// kRsFixHalo is left as it is, and unless it is in order already (one value
-// many times) the array is sent to the rescue passes: each of its keys is
-// compared with the one before, by the warp before for a chunk's first
-// kRsFixHalo keys and by the chunk's own warp from the next on.  One read of
+// kRsFixHalo is left as it is and entered in a list by the warp that sees its
+// first key.  The list matters only when one of those runs is out of order
+// (not one value many times): each of their keys is compared with the one
+// before, by the warp before for a chunk's first kRsFixHalo keys and by the
+// chunk's own warp from the next on.  One read of
 // the keys, bound by memory where runs are rare; warps work on their own, so
 // that one warp's loads run behind another's comparisons (a CTA-wide tile of
 // 4096 keys between barriers took 271 us for 2^26 random keys on a B200).
 constexpr int kRsFixThreads = 128, kRsFixPer = 8, kRsFixChunk = 32 * kRsFixPer, kRsFixHalo = 64;
 
 template <typename K, typename P>
-__global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *vals, uint32_t n, RsPlanWs *plan) {
+__global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *vals, uint32_t n, RsPlanWs *plan,
+                                                                     RsRunList list) {
   constexpr int WARPS = kRsFixThreads / 32, LEN = kRsFixChunk + kRsFixHalo, PER = LEN / 32;
   using V = typename std::conditional<has_payload<P>(), P, char>::type;
   grid_dependency_wait();
@@ -593,7 +619,17 @@ __global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *v
         rank += low[last] < l;
       }
       if (last - first >= kRsFixHalo) {  // (true of a run that reaches the halo's end)
-        if (i > first && low[i - 1] > l) plan->rescue = 1u;
+        if (i > first) {
+          if (low[i - 1] > l) plan->unordered = 1u;
+        } else {  // its first key
+          auto reaches = [&](unsigned int q) {  // key q of the run, counted from 0
+            return n - base - i > q && (unsigned int)(RadixKey<K>::to(kp[i + q]) >> 32) == u;
+          };
+          const bool longer = reaches(kRsRunWarp);
+          const unsigned int at = atomicAdd(&plan->runs[longer], 1u);
+          if (at >= list.room_for(longer, n) || (longer && reaches(kRsRunMax))) plan->too_many = 1u;
+          else *list.slot(longer, at) = (unsigned int)base + (unsigned int)i;
+        }
       } else if (first + rank != i) {
         s_to[warp][i] = (uint16_t)(first + rank);
         moves |= 1u << j;
@@ -623,9 +659,9 @@ __global__ void __launch_bounds__(kRsFixThreads, 10) rs_fix_kernel(K *keys, P *v
 // (two, where eight digits are counted) ever meet in a bank, however the
 // digits are distributed; a CTA adds its sums to the array's counts when its
 // run of tiles leaves the array.  128 KB of counters, one CTA of 1024 threads
-// an SM.  With a plan the first launch counts the digits that the passes
-// after it need and a second one, for the rescue, the rest.  The first also
-// clears the status rows that the first pass will publish in.
+// an SM.  With a plan it counts the digits that the passes after it need
+// (rs_late_kernel counts the rest for the rescue).  It also clears the status
+// rows that the first pass will publish in.
 constexpr int kRsHistThreads = 1024;
 constexpr size_t kRsHistSmemBytes = 128 * 1024;
 
@@ -701,23 +737,218 @@ __device__ __forceinline__ void rs_count_digits(const Src &src, unsigned int gro
 template <typename K, typename P, typename Src, int C>
 __global__ void __launch_bounds__(kRsHistThreads, 1) rs_hist_kernel(const __grid_constant__ Src src,
                                                                     unsigned int groups, unsigned int *hist,
-                                                                    uint4 *status, const RsPlanWs *plan,
-                                                                    bool rescue) {
+                                                                    uint4 *status, const RsPlanWs *plan) {
   extern __shared__ __align__(16) unsigned int rs_hist_smem[];
   for (int i = threadIdx.x; i < (int)(kRsHistSmemBytes / 16); i += kRsHistThreads)
     reinterpret_cast<uint4 *>(rs_hist_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
   grid_dependency_wait();
   const RsPlan p = rs_plan(plan, plan != nullptr ? src.group(0).n : 0);
-  if (rescue) {
-    if (p == kPlanRescue) rs_count_digits<K, P, Src, C, 0, 4>(src, groups, hist);
-    return;
-  }
   for (uint64_t i = (uint64_t)blockIdx.x * kRsHistThreads + threadIdx.x; i < (uint64_t)groups * (kRsBins / 4);
        i += (uint64_t)gridDim.x * kRsHistThreads)
     status[i] = make_uint4(0u, 0u, 0u, 0u);
   if constexpr (sizeof(K) == 4) rs_count_digits<K, P, Src, C, 0, 4>(src, groups, hist);
   else if (p == kPlanFull) rs_count_digits<K, P, Src, C, 0, 8>(src, groups, hist);
   else rs_count_digits<K, P, Src, C, 4, 4>(src, groups, hist);
+}
+
+// ---- what the fix kernel left: the long runs it listed, or the rescue's counts.
+//
+// A warp sorts a run of up to kRsRunWarp keys by counting: a key's place is the
+// number of keys below it, and of equal ones before it.  The keys go to the
+// temporaries (the run's own stretch of them; the passes are done with them)
+// and back.  Bound by instructions, about 3.5 a comparison.  A run that is in
+// order is passed over.
+template <typename K, typename P>
+__device__ __forceinline__ void rs_sort_run_warp(K *keys, P *vals, K *tk, P *tv, uint32_t len, uint32_t *low) {
+  constexpr int ITEMS = 4;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t i = lane; i < len; i += 32) low[i] = (uint32_t)RadixKey<K>::to(ld_cg(keys + i));
+  if (lane < ((0u - len) & 3u)) low[len + lane] = ~0u;  // not below any key, after all
+  __syncwarp();
+  bool down = false;
+  for (uint32_t i = lane; i + 1 < len; i += 32) down |= low[i] > low[i + 1];
+  if (!__any_sync(0xffffffffu, down)) return;
+  for (uint32_t first = lane; first - lane < len; first += 32 * ITEMS) {  // this lane's keys: first + 32 j
+    uint32_t l[ITEMS], rank[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      l[j] = first + 32 * j < len ? low[first + 32 * j] : 0u;
+      rank[j] = 0u;
+    }
+    for (uint32_t q = 0; q < len; q += 4) {
+      const uint4 x = *reinterpret_cast<const uint4 *>(low + q);
+      const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j)
+          rank[j] += (unsigned int)(xs[t] < l[j]) | ((unsigned int)(xs[t] == l[j]) & (unsigned int)(q + t < first + 32 * j));
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      if (first + 32 * j < len) {
+        tk[rank[j]] = ld_cg(keys + first + 32 * j);
+        if constexpr (has_payload<P>()) tv[rank[j]] = ld_cg(vals + first + 32 * j);
+      }
+    }
+  }
+  __syncwarp();
+  for (uint32_t i = lane; i < len; i += 32) {
+    keys[i] = ld_cg(tk + i);
+    if constexpr (has_payload<P>()) vals[i] = ld_cg(tv + i);
+  }
+}
+
+// A CTA sorts a longer run by the four lower digits, a tile at a time: ranked
+// and staged as in the passes, each digit's run written to where the run's own
+// counts and its tiles before put it, to and fro between the array and the
+// temporaries.  Bound by latency: a tile's load, ranking and barriers, 4 to 5
+// us each.
+constexpr int kRsRunItems = 8, kRsRunTile = kRsHistThreads * kRsRunItems;
+template <typename K, typename P>
+__device__ __forceinline__ void rs_sort_run(K *keys, P *vals, K *tk, P *tv, uint32_t len) {
+  constexpr int TH = kRsHistThreads, ITEMS = kRsRunItems, WARPS = TH / 32, WARP_KEYS = 32 * ITEMS;
+  constexpr size_t VOFF = sizeof(K) * kRsRunTile;
+  static_assert(VOFF + (size_t)payload_bytes<P>() * kRsRunTile <= kRsHistSmemBytes, "the tile fits");
+  extern __shared__ __align__(16) unsigned int rs_hist_smem[];
+  unsigned char *const smem = reinterpret_cast<unsigned char *>(rs_hist_smem);
+  K *const sk = reinterpret_cast<K *>(smem);  // the tile in digit order
+  P *const sv = reinterpret_cast<P *>(smem + VOFF);
+  __shared__ __align__(16) uint16_t s_whist[WARPS][kRsBins];  // per-warp digit counters, then staging starts (both x4)
+  __shared__ unsigned int s_at[4][kRsBins];  // counts of the four digits, then where a digit's next key goes
+  __shared__ unsigned int s_dst[kRsBins];    // output position of staged position 0 for digit d
+  __shared__ unsigned int s_scan[kRsBins / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the ranking tables lie in the staging area, which is written after every warp has ranked its keys
+  unsigned char *const tables = smem + (256u - (smem_addr(smem) & 255u));
+  const RsRanker ranker(tables + warp * 512, tables + WARPS * 512 + warp * 128);
+  uint4 *const mine = reinterpret_cast<uint4 *>(&s_whist[warp][0]) + lane;  // a warp clears its own counters
+  *mine = make_uint4(0u, 0u, 0u, 0u);
+  (&s_at[0][0])[tid] = 0u;
+  __syncthreads();
+  bool down = false;
+  for (uint32_t i = tid; i < len; i += TH) {
+    const uint32_t l = (uint32_t)RadixKey<K>::to(ld_cg(keys + i));
+#pragma unroll
+    for (int d = 0; d < 4; ++d) atomicAdd(&s_at[d][(l >> (8 * d)) & 0xffu], 1u);
+    if (i > 0) down |= (uint32_t)RadixKey<K>::to(ld_cg(keys + i - 1)) > l;
+  }
+  if (!__syncthreads_or(down)) return;
+  for (int pass = 0; pass < 4; ++pass) {
+    const K *const in_k = (pass & 1) ? tk : keys;
+    const P *const in_v = (pass & 1) ? tv : vals;
+    K *const out_k = (pass & 1) ? keys : tk;
+    P *const out_v = (pass & 1) ? vals : tv;
+    if (tid < kRsBins) {
+      unsigned int all;
+      s_at[pass][tid] = rs_scan_digits(s_at[pass][tid], s_scan, all);
+    }
+    __syncthreads();
+    for (uint32_t base = 0; base < len; base += kRsRunTile) {
+      const int count = (int)(len - base < (uint32_t)kRsRunTile ? len - base : (uint32_t)kRsRunTile);
+      const int warps = (count + WARP_KEYS - 1) / WARP_KEYS;  // that have keys
+      auto elem = [&](int j) { return warp * WARP_KEYS + j * 32 + lane; };
+      K k[ITEMS];
+      P v[ITEMS];
+      uint32_t dig4[ITEMS / 4], rank2[ITEMS / 2];
+      if (warp < warps) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+          const bool ok = elem(j) < count;
+          k[j] = ok ? ld_cg(in_k + base + elem(j)) : K();
+          if constexpr (has_payload<P>()) v[j] = ok ? ld_cg(in_v + base + elem(j)) : P();
+        }
+        // past the run's end the digit is 255: those items stay last
+#pragma unroll
+        for (int i = 0; i < ITEMS / 4; ++i) dig4[i] = rs_digits4(k + 4 * i, pass);
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j)
+          if (elem(j) >= count) dig4[j >> 2] |= 0xffu << (8 * (j & 3));
+        ranker.rank<ITEMS>(s_whist[warp], dig4, rank2);
+      }
+      __syncthreads();
+      if (tid < kRsBins) {
+        unsigned int cnt = 0, all;
+        for (int w = 0; w < warps; ++w) cnt += s_whist[w][tid];
+        const unsigned int excl = rs_scan_digits(cnt, s_scan, all);
+        unsigned int run = excl;
+        for (int w = 0; w < warps; ++w) {
+          const unsigned int c = s_whist[w][tid];
+          s_whist[w][tid] = (uint16_t)run;
+          run += c;
+        }
+        cnt >>= 2;
+        if (tid == kRsBins - 1) cnt -= (unsigned int)(warps * WARP_KEYS - count);
+        const unsigned int at = s_at[pass][tid];
+        s_dst[tid] = at - (excl >> 2);
+        s_at[pass][tid] = at + cnt;
+      }
+      __syncthreads();
+      if (warp < warps) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+          const uint32_t d = (dig4[j >> 2] >> (8 * (j & 3))) & 0xffu;
+          const uint32_t pos = (s_whist[warp][d] + ((rank2[j >> 1] >> (16 * (j & 1))) & 0xffffu)) >> 2;
+          sk[pos] = k[j];
+          if constexpr (has_payload<P>()) sv[pos] = v[j];
+        }
+        __syncwarp();
+        *mine = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncthreads();
+      for (int p = tid; p < count; p += TH) {
+        const K key = sk[p];
+        const uint32_t to = s_dst[rs_digit1(key, pass)] + (uint32_t)p;
+        if (to < len) {
+          out_k[to] = key;
+          if constexpr (has_payload<P>()) out_v[to] = sv[p];
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+template <typename K, typename P, typename Src, int C>
+__global__ void __launch_bounds__(kRsHistThreads, 1) rs_late_kernel(const __grid_constant__ Src src,
+                                                                    unsigned int groups, unsigned int *hist,
+                                                                    const RsPlanWs *plan, RsRunList list) {
+  extern __shared__ __align__(16) unsigned int rs_hist_smem[];
+  static_assert((size_t)kRsHistThreads / 32 * kRsRunWarp * 4 <= kRsHistSmemBytes, "a warp's run each");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < (int)(kRsHistSmemBytes / 16); i += kRsHistThreads)
+    reinterpret_cast<uint4 *>(rs_hist_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  grid_dependency_wait();
+  const RsGroup<K, P> gr = src.group(0);
+  const RsPlan p = rs_plan(plan, gr.n);
+  if (p == kPlanRescue) rs_count_digits<K, P, Src, C, 0, 4>(src, groups, hist);
+  if (p != kPlanUpper || ld_cg(&plan->unordered) == 0u) return;
+  auto upper = [&](uint64_t i) { return (unsigned int)(RadixKey<K>::to(ld_cg(gr.keys + i)) >> 32); };
+  const unsigned int longer = ld_cg(&plan->runs[1]), shorter = ld_cg(&plan->runs[0]);
+  for (unsigned int r = blockIdx.x; r < longer; r += gridDim.x) {
+    const uint64_t start = ld_cg(list.slot(true, r));
+    const unsigned int u = upper(start);
+    auto in_run = [&](uint32_t q) { return start + q < gr.n && upper(start + q) == u; };
+    // its length: whole steps, then the keys of the step that is not
+    constexpr uint32_t STEP = kRsRunMax / kRsHistThreads;
+    uint32_t len = STEP * (uint32_t)__syncthreads_count(in_run(threadIdx.x * STEP + STEP - 1));
+    len += (uint32_t)__syncthreads_count(threadIdx.x < STEP && in_run(len + threadIdx.x));
+    rs_sort_run<K, P>(gr.keys + start, has_payload<P>() ? gr.vals + start : nullptr, gr.tk + start,
+                      has_payload<P>() ? gr.tv + start : nullptr, len);
+    __syncthreads();
+  }
+  // one warp of each CTA first
+  for (unsigned int r = warp * gridDim.x + blockIdx.x; r < shorter; r += gridDim.x * (kRsHistThreads / 32)) {
+    const uint64_t start = ld_cg(list.slot(false, r));
+    const unsigned int u = upper(start);
+    auto in_run = [&](uint32_t q) { return start + q < gr.n && upper(start + q) == u; };
+    constexpr uint32_t STEP = kRsRunWarp / 32;
+    uint32_t len = STEP * (uint32_t)__popc(__ballot_sync(0xffffffffu, in_run(lane * STEP + STEP - 1)));
+    if (len < kRsRunWarp) len += (uint32_t)__popc(__ballot_sync(0xffffffffu, in_run(len + lane)));
+    rs_sort_run_warp<K, P>(gr.keys + start, has_payload<P>() ? gr.vals + start : nullptr, gr.tk + start,
+                           has_payload<P>() ? gr.tv + start : nullptr, len, rs_hist_smem + warp * kRsRunWarp);
+    __syncwarp();
+  }
 }
 
 // ---- one pass: stable scatter by digit (keys -> temporaries on even passes,
@@ -1400,14 +1631,18 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
                                     zero_vecs)) != BK_OK)
     return st;
   RsPlanWs *plan = nullptr;
-  int fix_ctas = 0;
+  unsigned fix_ctas = 0, late_ctas = 0;
   if constexpr (kPlanned) {
     if (src.n >= kRsPlanMinN) {
       plan = reinterpret_cast<RsPlanWs *>(ws + L.plan);
       struct FixSite {};
       host::KernelSetup fs;
       if ((st = host::kernel_setup<FixSite>(rs_fix_kernel<K, P>, kRsFixThreads, 0, &fs)) != BK_OK) return st;
-      fix_ctas = (int)fs.resident_ctas;
+      fix_ctas = (unsigned)fs.resident_ctas;
+      struct LateSite {};
+      if ((st = host::kernel_setup<LateSite>(rs_late_kernel<K, P, Src, C>, kRsHistThreads, kRsHistSmemBytes, &fs)) != BK_OK)
+        return st;
+      late_ctas = (unsigned)fs.resident_ctas;
       st = host::launch_overlapped(rs_sample_kernel<K>, kRsSampleCtas, kRsSampleThreads, 0, stream, 1,
                                    (const K *)src.keys, (uint32_t)src.n,
                                    reinterpret_cast<unsigned int *>(ws + L.samples), plan);
@@ -1416,11 +1651,9 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
   }
   const uint64_t tiles = L.groups * C;
   const unsigned hist_ctas = (unsigned)(tiles < hs.resident_ctas ? tiles : hs.resident_ctas);
-  auto count = [&](bool rescue) {
-    return host::launch_overlapped(hist_kern, hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream, 1, src, groups, hist,
-                                   reinterpret_cast<uint4 *>(ws + L.status[0]), (const RsPlanWs *)plan, rescue);
-  };
-  if ((st = count(false)) != BK_OK) return st;
+  st = host::launch_overlapped(hist_kern, hist_ctas, kRsHistThreads, kRsHistSmemBytes, stream, 1, src, groups, hist,
+                               reinterpret_cast<uint4 *>(ws + L.status[0]), (const RsPlanWs *)plan);
+  if (st != BK_OK) return st;
   const unsigned used = groups < (unsigned)clusters ? groups : (unsigned)clusters;
   // L2 prefetch distance: the table's number of residencies ahead (0: none)
   const tune::Knobs kn = tune::knobs_for(tune::kSort, RsCfg<K, P>::BYTES, L.groups * C * RsCfg<K, P>::TILE);
@@ -1434,9 +1667,14 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
     if (st != BK_OK) return st;
     if constexpr (kPlanned) {
       if (plan != nullptr && p == 3) {
-        st = host::launch_overlapped(rs_fix_kernel<K, P>, (unsigned)fix_ctas, kRsFixThreads, 0, stream, 1, src.keys,
-                                     src.vals, (uint32_t)src.n, plan);
-        if (st != BK_OK || (st = count(true)) != BK_OK) return st;
+        // the rows that launch 3 published in and launch 4 clears
+        const RsRunList list{reinterpret_cast<unsigned int *>(ws + L.status[1]), groups * (unsigned)kRsBins};
+        st = host::launch_overlapped(rs_fix_kernel<K, P>, fix_ctas, kRsFixThreads, 0, stream, 1, src.keys, src.vals,
+                                     (uint32_t)src.n, plan, list);
+        if (st != BK_OK) return st;
+        st = host::launch_overlapped(rs_late_kernel<K, P, Src, C>, late_ctas, kRsHistThreads, kRsHistSmemBytes, stream, 1,
+                                     src, groups, hist, (const RsPlanWs *)plan, list);
+        if (st != BK_OK) return st;
       }
     }
   }

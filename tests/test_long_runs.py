@@ -83,3 +83,74 @@ def test_runs_about_as_long_as_the_longest_sorted_in_place(cuda, length):
         for at in range(1, length):
             case.check(_one_break(length, at, cuda))
     assert bulk_b200.workspace_status() == 0
+
+
+def _outside_the_sample(n, cuda):
+    """The positions that the sample (rs_sample_kernel: 32 windows of 65,536 keys) does not read."""
+    outside = torch.ones(n, dtype=torch.bool, device=cuda)
+    for cta in range(32):
+        h = (cta + 1) * 0x9E3779B1 % (1 << 32)
+        h = (h ^ h >> 15) * 0x85EBCA6B % (1 << 32)
+        h = (h ^ h >> 13) * 0xC2B2AE35 % (1 << 32)
+        h ^= h >> 16
+        window = h * (n - 65536) >> 32
+        outside[window:window + 65536] = False
+    return outside.nonzero()[:, 0]
+
+
+def _check_runs(tag, value, runs, cuda, low_bits=32, n=N, unseen=False):
+    """Runs of the given lengths at random places (unseen: that the sample does not read) among keys of distinct
+    upper halves, lower halves random."""
+    g = torch.Generator(device=cuda).manual_seed(len(runs) + runs[0])
+    upper = torch.randperm(n, device=cuda, generator=g)
+    low = torch.randint(0, 1 << low_bits, (n,), device=cuda, generator=g)
+    places = _outside_the_sample(n, cuda) if unseen else torch.arange(n, device=cuda)
+    places = places[torch.randperm(places.numel(), device=cuda, generator=g)]
+    lengths = torch.tensor(runs, device=cuda)
+    members = places[:int(lengths.sum())]
+    assert members.numel() == int(lengths.sum())
+    upper[members] = torch.repeat_interleave(n + torch.arange(len(runs), device=cuda) * 3, lengths)
+    if tag == "i64":
+        upper -= n
+    elif tag == "f64":
+        upper += 0x3FF00000
+    keys = (upper << 32) | low
+    if tag == "f64":  # a run at zero: the two zeros tie, the least numbers share their upper half
+        zero = places[-300:]
+        keys[zero[:100]] = -(1 << 63)
+        keys[zero[100:200]] = 0
+        keys[zero[200:]] = low[zero[200:]]
+    dtype = {"u64": torch.uint64, "i64": torch.int64, "f64": torch.float64}[tag]
+    want, order = torch.sort(keys.view(torch.float64) if tag == "f64" else keys, stable=True)
+    want = keys[order]
+    if value is None:
+        got = bulk_b200.stable_sort_by_key(keys.clone().view(dtype))
+    else:
+        got, vals = bulk_b200.stable_sort_by_key(keys.clone().view(dtype), torch.arange(n, device=cuda).to(value))
+        assert torch.equal(vals, order.to(value)), (runs[:3], len(runs))
+    assert torch.equal(got.view(torch.int64), want), (runs[:3], len(runs))
+    assert bulk_b200.workspace_status() == 0
+
+
+@pytest.mark.parametrize("tag,value", [("u64", torch.int32), ("i64", None), ("f64", torch.int64)])
+def test_runs_sorted_by_a_warp_or_a_cta(cuda, tag, value):
+    # a warp's, around its last key and its rounds of 128; a CTA's, around a warp's share, a tile and several
+    for length in (65, 66, 67, 68, 127, 128, 129, 255, 256, 257, 511, 513, 8191, 8192, 8193, 16385, 50_000):
+        _check_runs(tag, value, [length], cuda)
+        _check_runs(tag, value, [length], cuda, low_bits=1)
+    _check_runs(tag, value, [65, 9000, 70, 8192, 300, 20_000, 66, 256, 257], cuda)
+    _check_runs(tag, value, [131_071, 66], cuda, unseen=True)
+    _check_runs(tag, value, [131_072, 5000, 5000], cuda, unseen=True)
+
+
+@pytest.mark.parametrize("tag,value", [("u64", torch.int32), ("i64", None), ("f64", torch.int64)])
+def test_longer_and_more_runs_than_those(cuda, tag, value):
+    _check_runs(tag, value, [131_073], cuda, unseen=True)
+    _check_runs(tag, value, [300_000, 100], cuda, unseen=True)
+    n = 1 << 24
+    _check_runs(tag, value, [258] * 30_000, cuda, n=n, unseen=True)
+    tile = 3456 if value == torch.int64 else 4608  # the list: a word a digit and group of four tiles, less one in 256 keys
+    room = (n + 4 * tile - 1) // (4 * tile) * 256 - n // 256
+    for count in (10_000, room - 1, room, room + 1):
+        if count * 65 < 14_000_000:
+            _check_runs(tag, value, [65] * count, cuda, n=n, unseen=True)

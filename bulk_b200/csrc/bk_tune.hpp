@@ -9,7 +9,8 @@
 //   ctas_per_sm  persistent / grid-stride CTAs per SM (the grid is that many
 //                times the SM count, or the tile count when smaller);
 //   prefetch     L2 prefetch distance in residencies (0: none; read by the
-//                radix sort, whose tiles are not persistent).
+//                radix sort's passes, whose clusters take groups of tiles in
+//                turn: a group that many rounds of all clusters ahead).
 // Size classes: 0 below 2^16 elements, 1 below 2^20, 2 below 2^24, 3 from
 // 2^24.  A missing entry takes the op's default.  A process-wide override
 // per (op, element bytes, size class) lets the tuning procedure try knobs

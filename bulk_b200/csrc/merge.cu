@@ -534,11 +534,12 @@ int merge_launch(const K *a, const P *av, uint64_t na, const K *b, const P *bv, 
   const unsigned long long limit = dbg.spin_limit_ns ? dbg.spin_limit_ns : host::kDefaultSpinLimitNs;
   // Many tiles a CTA: a partition kernel first, whose splits cost the loader
   // nothing; few: the loader finds them (see merge_kernel).  Measured on a
-  // B200, partition / loader: f32/u32 2 x 2^18 17.4 / 13.0 us, 2 x 2^22 46.1 /
-  // 37.9, 2 x 2^24 (18 tiles a CTA) 113.7 / 113.6, 2 x 2^25 201.7 / 206.8;
-  // f64/u32 2 x 2^21 39.8 / 33.6, 2 x 2^22 (9 a CTA) 62.5 / 62.3, 2 x 2^24
-  // 169 / 181; f64 2 x 2^22 52.2 / 47.1, 2 x 2^24 136.2 / 135.2; f32 2 x 2^18
-  // 15.3 / 11.1, 2 x 2^26 273 / 262 (keys of 4 bytes alone never need it).
+  // B200, partition / loader: i32/u32 2 x 2^18 13.3 / 9.7 us, 2 x 2^22 38.9 /
+  // 35.3, 2 x 2^23 (9 tiles a CTA) random 60.4 / 65.9 and of few values 89.1 /
+  // 84.5, 2 x 2^24 (18) 105 / 111; f64/u32 2 x 2^21 33.8 / 31.2, 2 x 2^22 (9)
+  // 51.2 / 57.9, 2 x 2^24 163 / 178; f64 2 x 2^22 (9) 44.0 / 43.5, 2 x 2^23
+  // 70.6 / 72.2; i32 2 x 2^18 11.2 / 8.7, 2 x 2^26 257 / 256 (keys of 4 bytes
+  // alone never need it).
   constexpr uint64_t kPerCta = C::PB == 0 ? (sizeof(K) == 4 ? ~0ull : 16) : (sizeof(K) == 4 ? 16 : 8);
   // With a partition kernel the CTAs' tiles are interleaved, so that all of
   // them read and write close to one another; 4-byte keys from 32 tiles a CTA

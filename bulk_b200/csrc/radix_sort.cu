@@ -36,7 +36,7 @@ namespace bk {
 constexpr int kRsBins = 256;                    // 8-bit digits
 constexpr uint64_t kRsMaxN = 1ull << 30;
 constexpr int kRsBatchMax = 256;
-constexpr int kRsWindow = 32;                   // earlier groups read in one look-back round
+constexpr int kRsWindow = 32;                   // words a lane of the scout reads in one look-back round
 
 // Order-preserving map of a key to an unsigned integer.
 template <typename K>
@@ -507,7 +507,9 @@ __global__ void rs_zero_kernel(uint4 *p, uint32_t vecs) {
 // and enters its upper half in a table of values seen (zeroed before; a zero
 // half is counted apart).  Windows, because reading 16,384 keys all over 2^26
 // costs their address translation; 128 keys apart, so that a sorted array's
-// runs that are short enough to be sorted in place rarely count.
+// runs that are short enough to be sorted in place rarely count.  The positions
+// come from MurmurHash3's 32-bit finaliser, the table's slots from Fibonacci
+// hashing (both published).
 template <typename K>
 __global__ void __launch_bounds__(kRsSampleThreads) rs_sample_kernel(const K *keys, uint32_t n, unsigned int *table,
                                                                      RsPlanWs *plan) {
@@ -962,12 +964,13 @@ __global__ void __launch_bounds__(kRsHistThreads, 1) rs_late_kernel(const __grid
 // (its AGGREGATE) and, once known, the end position (its PREFIX), one 32-bit
 // word each: a flag in the two top bits and the value below (n < 2^30).
 //
-// The look-back reads kRsWindow earlier groups in one round, one thread a
-// digit.  A per-tile look-back that walks one predecessor a round trip does
-// not keep up at this rate (a pass runs through 60 tiles of 4096 keys a
-// microsecond and a round trip takes most of one); groups of eight tiles and
-// rounds of 32 groups do, and cost an eighth of the traffic (a round reads
-// 32 KB per 32,768 keys).
+// The look-back reads 16 earlier groups in one round (eight where a group has
+// two tiles): kRsWindow words a lane of the scout warp, for its two digits
+// (four).  A look-back by single tiles that walks one predecessor a round trip
+// does not keep up: a pass runs through 30 tiles of 6656 pairs a microsecond
+// (2^26 u32/u32 on a B200), and a round trip takes most of one.  Groups of four
+// tiles and rounds of 16 groups do, and a round reads 16 KB for the 208 KB of
+// pairs of a group.
 //
 // A CTA's loop is pipelined by one tile: tile i + 1 is ranked and its counts
 // are sent before tile i, staged in shared memory in digit order, is written
@@ -1537,9 +1540,10 @@ inline int rs_group_ctas(const uint64_t *sizes, uint32_t count) {
 }
 
 // Workspace (after the 256-byte header): every array's key and payload
-// temporaries; zeroed before each sort: the arrays' digit counts and the
-// passes' tickets and a planned sort's sample; two buffers of status rows (one word a digit and group),
-// of which each pass publishes in one and clears the other.
+// temporaries; zeroed before each sort: the arrays' digit counts, the passes'
+// tickets and a planned sort's decision and sample; two buffers of status rows
+// (one word a digit and group), of which each pass publishes in one and clears
+// the other.
 template <typename K, typename P>
 struct RsLayout {
   size_t tmp, hist, tickets, plan, samples, zero_bytes, status[2], total;
@@ -1655,7 +1659,7 @@ int radix_sort_run(const Src &src, const RsLayout<K, P> &L, char *ws, cudaStream
                                reinterpret_cast<uint4 *>(ws + L.status[0]), (const RsPlanWs *)plan);
   if (st != BK_OK) return st;
   const unsigned used = groups < (unsigned)clusters ? groups : (unsigned)clusters;
-  // L2 prefetch distance: the table's number of residencies ahead (0: none)
+  // L2 prefetch distance: the table's number of rounds of all clusters ahead (0: none)
   const tune::Knobs kn = tune::knobs_for(tune::kSort, RsCfg<K, P>::BYTES, L.groups * C * RsCfg<K, P>::TILE);
   const unsigned ahead = used * (unsigned)kn.prefetch;
   const int launches = plan != nullptr ? 12 : rs_passes<K>();

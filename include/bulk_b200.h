@@ -222,7 +222,8 @@ BK_API int bk_merge_by_key_f64_u64(const double *a_keys, const uint64_t *a_vals,
  * stable order is unique, so the result is the reference's whichever way it
  * is computed: a stable LSD radix sort below 2^30 elements (up to 4096 keys in
  * one thread block, up to 131,072 as one launch of one thread-block cluster,
- * above that as one counting launch and one launch a pass), block sort and merge-path passes from 2^30 on.  Keys
+ * above that as a counting launch and a launch a pass, with a few more for
+ * 8-byte keys from 2^22 on), block sort and merge-path passes from there on.  Keys
  * must not be NaN.  bk_sort_keys_* sorts keys alone. */
 BK_API int bk_sort_keys_i32(int32_t *keys, uint64_t n, void *d_ws, size_t ws_bytes, bk_stream_t stream);
 BK_API int bk_sort_keys_u32(uint32_t *keys, uint64_t n, void *d_ws, size_t ws_bytes, bk_stream_t stream);
